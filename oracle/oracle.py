@@ -32,9 +32,14 @@ def ref_root() -> str:
     return os.environ.get("REF_ROOT") or os.path.normpath(os.path.join(HERE, "..", "..", "reference"))
 
 
+def ref_sources() -> bool:
+    """Whether the reference's sources are there (an empty checkout is not)."""
+    return os.path.isfile(os.path.join(ref_root(), "src", "ckernel.cpp"))
+
+
 def build(ref: bool = False) -> None:
     """Compile the oracle (and oracle/_ref when the reference tree exists)."""
-    target = "ref" if (ref and os.path.isdir(ref_root())) else "all"
+    target = "ref" if (ref and ref_sources()) else "all"
     subprocess.run(["make", "-s", "-C", HERE, target, f"REF_ROOT={ref_root()}"], check=True)
 
 
