@@ -25,6 +25,7 @@
 #include "bv_knn.cuh"
 #include "bv_llh_big.cuh"
 #include "bv_llh_fp64.cuh"
+#include "bv_llh_lean.cuh"
 #include "bv_llh_mixed.cuh"
 #include "bv_reduce.cuh"
 
@@ -61,13 +62,12 @@ static void (*const llh_fp64_big_kernel3)(LlhArgs) = llh_fp64_kernel_t<true, tru
 
 // The streamed (left-looking, panels through L2) path run by small CTAs,
 // several per SM, so that the pivot chains of several blocks overlap on one
-// SM: NT threads per CTA, RC rows per streamed chunk, MINB CTAs per SM.
-template <int NT, int RC, int MINB, int NS, bool kXYZ3, bool kBulk>
+// SM: NT threads per CTA, MINB CTAs per SM, GEN the entries' kind.
+template <int NT, int MINB, int GEN>
 __global__ void __launch_bounds__(NT, MINB) llh_lean_kernel_t(LlhArgs a)
 {
     extern __shared__ __align__(128) double smem[];
     __shared__ LeanShared sh;
-    const MaternParams mp = *a.mp;
     const int tid = threadIdx.x;
     const int task_end = a.task_count ? min(a.task_end, *a.task_count) : a.task_end;
     double *slab = a.gslab + (size_t)blockIdx.x * a.gslab_stride;
@@ -86,58 +86,29 @@ __global__ void __launch_bounds__(NT, MINB) llh_lean_kernel_t(LlhArgs a)
                 a.block_status[b] = a.status_or;
             }
         } else {
-            process_block_big<NT, RC, LeanShared, NS, kXYZ3, kBulk>(
-                a, mp, b, reinterpret_cast<unsigned char *>(smem), slab, sh);
+            process_block_lean<NT, GEN>(a, a.mp, b, reinterpret_cast<unsigned char *>(smem), slab, sh);
         }
         __syncthreads();
     }
 }
 
 struct LeanVariant {
-    void (*kernel)(LlhArgs);   // 2-D locations
-    void (*kernel3)(LlhArgs);  // with a third coordinate
-    int threads, rc, ns;
-    bool bulk;  // the whole matrix generated into the slab before the factorization
+    void (*kernel[3])(LlhArgs);  // by LeanGen
+    int threads;
 };
-#define BV_LEAN(NT, RC, MINB, NS, BULK)                                                              \
-    {llh_lean_kernel_t<NT, RC, MINB, NS, false, BULK>, llh_lean_kernel_t<NT, RC, MINB, NS, true, BULK>, \
-     NT, RC, NS, BULK}
-// The left-looking update reads the earlier panels straight from the slab
-// (no staging), so the CTAs can be small and several blocks share an SM.
-// Kernel ms, n = 200k uniform, bc = 20k, nu = 1.5: the persistent kernel;
-// then 96-thread CTAs x5 per SM, 160 x3 and 256 x2 generating panel by panel
-// (the first three variants; the whole-matrix generation, the last three,
-// wins only where the generation is expensive: general nu):
-//   cs =  40 (M <=  74):  2.54 /  0.80 /  1.00 /  1.35
-//   cs =  80 (M <= 114):  4.48 /  2.02 /  2.16 /  2.58
-//   cs = 120 (M <= 154):  6.88 /  4.13 /  4.01 /  4.40
-//   cs = 160 (M <= 194): 10.00 /  8.89 /  6.62 /  7.04
-//   cs = 200 (M <= 234): 13.70 / 14.79 / 10.73 / 10.78
-//   cs = 240 (M <= 274): 26.23 / 28.65 / 18.41 / 15.43
-//   cs = 300 (M <= 334): 40.94 / 47.85 / 30.23 / 25.35
-// At the headline shape (n = 1M, cs = 200, nu = 2.5, largest M 240):
-// 68.0 / 73.3 / 53.2 / 53.5; at the general-nu stress shape (2M points,
-// cs = 300, nu = 0.8) 256 x2 generating the whole matrix first, 526 ms,
-// against 537 panel by panel.  128 x4 (four CTAs while two panels of
-// M <= ~200 fit) is the fastest up to M ~ 170 (cs = 40 / 80 / 120: 0.78 /
-// 1.98 / 3.86).  Larger CTAs spill (288 or 320 threads x2, 192 x3, 160 x4)
-// or run one block per SM (512 x1); 128 x3 and 192 x2 lost everywhere.
-// All give the same bits (the per-element operations do not
-// depend on the CTA size or the generation mode), so bv_opts.tune may pick
-// any of them.
+#define BV_LEAN(NT, MINB)                                                                          \
+    {{llh_lean_kernel_t<NT, MINB, kGenClosed>, llh_lean_kernel_t<NT, MINB, kGenGeneral>,          \
+      llh_lean_kernel_t<NT, MINB, kGenXYZ>}, NT}
+// The table's three sizes and three others (lean_table_threads has the
+// measurements).  All give the same bits, so bv_opts.tune may pick any.
 static const LeanVariant kLeanVariants[] = {
-    BV_LEAN(96, 64, 5, 0, false),
-    BV_LEAN(160, 64, 3, 0, false),
-    BV_LEAN(256, 64, 2, 0, false),
-    BV_LEAN(128, 64, 4, 0, false),
-    BV_LEAN(160, 64, 3, 0, true),
-    BV_LEAN(256, 64, 2, 0, true),
+    BV_LEAN(96, 4), BV_LEAN(160, 3), BV_LEAN(256, 2), BV_LEAN(128, 3), BV_LEAN(160, 2), BV_LEAN(256, 1),
 };
 constexpr int kNumLean = (int)(sizeof(kLeanVariants) / sizeof(kLeanVariants[0]));
-static int lean_variant(int max_m)
+static int lean_variant(int gen, int max_m, size_t blocks)
 {
-    const int t = lean_table_threads(max_m);
-    return t == 128 ? 3 : (t == 160 ? 1 : 2);  // the panel-by-panel variants
+    const int t = lean_table_threads(gen, max_m, blocks);
+    return t == 96 ? 0 : (t == 128 ? 3 : 2);
 }
 
 static thread_local char g_err[1024] = "";
@@ -187,7 +158,7 @@ struct bv_handle {
     bool mixed_lean = false;        // mixed path: the FP64 pass runs the streamed kernel (last launch)
     // The streamed launch's order positions and largest M, its CTA size
     // (kLeanVariants index; -1: from the table), and the tuner's record.
-    int lean_begin = 0, lean_end = 0, lean_m = 0, lean_choice = -1, lean_threads = 0, lean_vi = -1;
+    int lean_begin = 0, lean_end = 0, lean_m = 0, lean_choice = -1;
     bool tuned = false;
     double tune_ms[kNumLean] = {};
     MaternParams *d_mp = nullptr;
@@ -204,18 +175,23 @@ struct bv_handle {
     size_t smem_bytes = 0;
     int grid = 0;
     int block_threads = kThreads;
-    struct Launch {
-        int begin, end, grid;
-        void (*kernel)(LlhArgs);
+    struct Kernel {
+        void (*fn)(LlhArgs);
         int threads;
+        int grid;
         size_t smem;
+        int variant;  // kLeanVariants index, -1: the persistent kernel
+    };
+    struct Launch {
+        int begin, end;
         double *slab;
         size_t slab_stride;
+        Kernel k[2];  // closed-form nu, general nu
     };
     std::vector<Launch> launches;
     cudaStream_t stream = nullptr;
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t gexec = nullptr;
+    cudaGraph_t graph[2] = {nullptr, nullptr};  // closed-form nu, general nu
+    cudaGraphExec_t gexec[2] = {nullptr, nullptr};
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, evk0 = nullptr, evk1 = nullptr;
     cudaStream_t own_stream = nullptr;  // the handle's stream; `stream` may be a caller's
     // status
@@ -229,8 +205,10 @@ static void handle_free(bv_handle *h)
     int prev = 0;
     cudaGetDevice(&prev);
     cudaSetDevice(h->device);
-    if (h->gexec) cudaGraphExecDestroy(h->gexec);
-    if (h->graph) cudaGraphDestroy(h->graph);
+    for (int g = 0; g < 2; ++g) {
+        if (h->gexec[g]) cudaGraphExecDestroy(h->gexec[g]);
+        if (h->graph[g]) cudaGraphDestroy(h->graph[g]);
+    }
     if (h->ev0) cudaEventDestroy(h->ev0);
     if (h->ev1) cudaEventDestroy(h->ev1);
     if (h->evk0) cudaEventDestroy(h->evk0);
@@ -424,39 +402,48 @@ static int order_m(const bv_handle *h, int t)
 // largest block has M = max_m.
 static int plan_lean_launch(bv_handle *h, const cudaDeviceProp &prop, int begin, int end, int max_m)
 {
-    const int vi = h->lean_choice >= 0 ? h->lean_choice : lean_variant(max_m);
-    const LeanVariant &v = kLeanVariants[vi];
-    h->lean_vi = vi;
     h->lean_begin = begin;
     h->lean_end = end;
     h->lean_m = max_m;
-    h->lean_threads = v.threads;
-    void (*const kern)(LlhArgs) = h->nz ? v.kernel3 : v.kernel;
-    cudaFuncAttributes fa;
-    BV_CUDA_TRY(cudaFuncGetAttributes(&fa, kern));
     int optin = 0;
     BV_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
-    const size_t smem = big_layout(max_m, v.rc, h->nz, v.ns).total;
-    if (smem > (size_t)optin - fa.sharedSizeBytes) {
-        set_error("plan: blocks of M = %d exceed the streamed schedule's shared memory", max_m);
-        return BV_E_TOOLARGE;
+    bv_handle::Launch ln{begin, end, nullptr, (big_slab_doubles(max_m) + 31) & ~(size_t)31, {}};
+    int grid = 0;
+    for (int g = 0; g < 2; ++g) {
+        bv_handle::Kernel &k = ln.k[g];
+        const int gen = h->nz ? kGenXYZ : g;
+        k.variant = h->lean_choice >= 0 ? h->lean_choice : lean_variant(gen, max_m, (size_t)(end - begin));
+        const LeanVariant &v = kLeanVariants[k.variant];
+        k.fn = v.kernel[gen];
+        k.threads = v.threads;
+        k.smem = big_layout(max_m, 0, h->nz, 0).total;
+        cudaFuncAttributes fa;
+        BV_CUDA_TRY(cudaFuncGetAttributes(&fa, k.fn));
+        if (k.smem > (size_t)optin - fa.sharedSizeBytes) {
+            set_error("plan: blocks of M = %d exceed the streamed schedule's shared memory", max_m);
+            return BV_E_TOOLARGE;
+        }
+        // The cap is per kernel, not per handle: what the device allows, so
+        // that handles with different block sizes can coexist.
+        BV_CUDA_TRY(cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)((size_t)optin - fa.sharedSizeBytes)));
+        int occ = 0;
+        BV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k.fn, v.threads, k.smem));
+        if (occ < 1) {
+            set_error("plan: streamed kernel cannot be resident (smem %zu B)", k.smem);
+            return BV_E_TOOLARGE;
+        }
+        k.grid = std::min(prop.multiProcessorCount * occ, end - begin);
+        grid = std::max(grid, k.grid);
     }
-    BV_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int occ = 0;
-    BV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, v.threads, smem));
-    if (occ < 1) {
-        set_error("plan: streamed kernel cannot be resident (smem %zu B)", smem);
-        return BV_E_TOOLARGE;
-    }
-    const int grid = std::min(prop.multiProcessorCount * occ, end - begin);
-    const size_t stride = (big_slab_doubles(max_m) + 31) & ~(size_t)31;
-    const size_t bytes = stride * sizeof(double) * (size_t)grid;
+    const size_t bytes = ln.slab_stride * sizeof(double) * (size_t)grid;
     if (cudaMalloc(&h->d_slab_lean, bytes) != cudaSuccess) {
         cudaGetLastError();
         set_error("plan: cannot allocate %zu B of block slabs", bytes);
         return BV_E_NOMEM;
     }
-    h->launches.push_back({begin, end, grid, kern, v.threads, smem, h->d_slab_lean, stride});
+    ln.slab = h->d_slab_lean;
+    h->launches.push_back(ln);
     return BV_OK;
 }
 
@@ -487,8 +474,8 @@ static int plan_launches(bv_handle *h)
         int optin = 0;
         BV_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
         cudaFuncAttributes fa;
-        BV_CUDA_TRY(cudaFuncGetAttributes(&fa, kLeanVariants[2].kernel));
-        lean_limit = big_max_m_for_bytes((size_t)optin - fa.sharedSizeBytes, 64, h->nz, 0);
+        BV_CUDA_TRY(cudaFuncGetAttributes(&fa, kLeanVariants[2].kernel[kGenClosed]));
+        lean_limit = big_max_m_for_bytes((size_t)optin - fa.sharedSizeBytes, 0, h->nz, 0);
     }
     if ((sched == BV_SCHED_STREAMED || sched == BV_SCHED_AUTO) && h->opts.precision == BV_PREC_FP64)
         h->lean_max_m = lean_limit;
@@ -538,10 +525,13 @@ static int plan_launches(bv_handle *h)
             return BV_E_NOMEM;
         }
     }
+    auto persistent = [&](int begin, int end, int grid) {
+        const bv_handle::Kernel k{h->kernel, kThreads, grid, h->smem_bytes, -1};
+        h->launches.push_back({begin, end, h->d_slab, h->slab_stride, {k, k}});
+    };
     if (sched != BV_SCHED_BUCKETED) {
         if (split > 0)
-            h->launches.push_back({0, split, h->grid, h->kernel, kThreads, h->smem_bytes, h->d_slab,
-                                   h->slab_stride});
+            persistent(0, split, h->grid);
     } else {
         // One launch per size bucket of M (width 8), largest first.
         int b = 0;
@@ -549,8 +539,7 @@ static int plan_launches(bv_handle *h)
             const int bucket = order_m(h, b) / 8;
             int e = b;
             while (e < split && order_m(h, e) / 8 == bucket) ++e;
-            h->launches.push_back({b, e, std::min(h->grid, e - b), h->kernel, kThreads, h->smem_bytes,
-                                   h->d_slab, h->slab_stride});
+            persistent(b, e, std::min(h->grid, e - b));
             b = e;
         }
     }
@@ -585,7 +574,21 @@ static cudaError_t record_timing(cudaEvent_t ev, cudaStream_t s)
 
 static int capture_graph(bv_handle *h);
 
-static int enqueue_eval(bv_handle *h, cudaStream_t s)
+// Kinds of evaluation that differ in their launches.
+static int graph_kinds(const bv_handle *h)
+{
+    for (const bv_handle::Launch &ln : h->launches)
+        if (ln.k[0].fn != ln.k[1].fn) return 2;
+    return 1;
+}
+
+static int eval_kind(const bv_handle *h)
+{
+    return (h->h_mp->nu_kind == kNuGeneral && graph_kinds(h) == 2) ? 1 : 0;
+}
+
+// One evaluation on stream s; kind: 0 a closed-form nu, 1 a general nu.
+static int enqueue_eval(bv_handle *h, cudaStream_t s, int kind)
 {
     BV_CUDA_TRY(cudaMemcpyAsync(h->d_mp, h->h_mp, sizeof(MaternParams), cudaMemcpyHostToDevice, s));
     BV_CUDA_TRY(cudaMemsetAsync(h->d_counters, 0, sizeof(unsigned) * std::max<size_t>(1, h->launches.size()), s));
@@ -643,7 +646,7 @@ static int enqueue_eval(bv_handle *h, cudaStream_t s)
             a.status_or = BV_ST_FP32_FALLBACK;
             a.gslab = ln.slab;
             a.gslab_stride = ln.slab_stride;
-            ln.kernel<<<ln.grid, ln.threads, ln.smem, s>>>(a);
+            ln.k[kind].fn<<<ln.k[kind].grid, ln.k[kind].threads, ln.k[kind].smem, s>>>(a);
             BV_CUDA_TRY(cudaGetLastError());
         } else if (h->owned > 0) {
             LlhArgs a = fp64_args(h->d_counters, h->mixed.fallback_list, 0, h->owned);
@@ -658,7 +661,7 @@ static int enqueue_eval(bv_handle *h, cudaStream_t s)
             LlhArgs a = fp64_args(h->d_counters + l, h->d_order, ln.begin, ln.end);
             a.gslab = ln.slab;
             a.gslab_stride = ln.slab_stride;
-            ln.kernel<<<ln.grid, ln.threads, ln.smem, s>>>(a);
+            ln.k[kind].fn<<<ln.k[kind].grid, ln.k[kind].threads, ln.k[kind].smem, s>>>(a);
             BV_CUDA_TRY(cudaGetLastError());
         }
     }
@@ -901,24 +904,30 @@ static int fill_params(bv_handle *h, const double *theta)
     return BV_OK;
 }
 
-// One evaluation captured into the handle's graph (replacing any earlier).
+// One evaluation of each kind captured into the handle's graphs (replacing
+// any earlier).  Without a streamed launch, or with a third coordinate, both
+// kinds run the same kernels and share the first graph.
 static int capture_graph(bv_handle *h)
 {
-    if (h->gexec) cudaGraphExecDestroy(h->gexec);
-    if (h->graph) cudaGraphDestroy(h->graph);
-    h->gexec = nullptr;
-    h->graph = nullptr;
-    BV_CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    const int erc = enqueue_eval(h, h->stream);
-    cudaGraph_t g = nullptr;
-    const cudaError_t ce = cudaStreamEndCapture(h->stream, &g);
-    if (erc || ce != cudaSuccess) {
-        if (g) cudaGraphDestroy(g);
-        if (!erc) set_error("graph capture: %s", cudaGetErrorString(ce));
-        return erc ? erc : BV_E_CUDA;
+    for (int g = 0; g < 2; ++g) {
+        if (h->gexec[g]) cudaGraphExecDestroy(h->gexec[g]);
+        if (h->graph[g]) cudaGraphDestroy(h->graph[g]);
+        h->gexec[g] = nullptr;
+        h->graph[g] = nullptr;
     }
-    h->graph = g;
-    BV_CUDA_TRY(cudaGraphInstantiate(&h->gexec, h->graph, 0));
+    for (int g = 0; g < graph_kinds(h); ++g) {
+        BV_CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+        const int erc = enqueue_eval(h, h->stream, g);
+        cudaGraph_t gr = nullptr;
+        const cudaError_t ce = cudaStreamEndCapture(h->stream, &gr);
+        if (erc || ce != cudaSuccess) {
+            if (gr) cudaGraphDestroy(gr);
+            if (!erc) set_error("graph capture: %s", cudaGetErrorString(ce));
+            return erc ? erc : BV_E_CUDA;
+        }
+        h->graph[g] = gr;
+        BV_CUDA_TRY(cudaGraphInstantiate(&h->gexec[g], h->graph[g], 0));
+    }
     return BV_OK;
 }
 
@@ -940,14 +949,14 @@ static int replan_lean(bv_handle *h, int vi)
 static int tune_lean(bv_handle *h)
 {
     h->tuned = true;
-    int best = h->lean_choice >= 0 ? h->lean_choice : lean_variant(h->lean_m);
+    int best = 0;
     double best_ms = 1e300;
     for (int vi = 0; vi < kNumLean; ++vi) {
         int rc = replan_lean(h, vi);
         if (rc) return rc;
         double t = 1e300;
         for (int rep = 0; rep < 2; ++rep) {
-            rc = enqueue_eval(h, h->stream);
+            rc = enqueue_eval(h, h->stream, eval_kind(h));
             if (rc) return rc;
             BV_CUDA_TRY(cudaStreamSynchronize(h->stream));
             float kms = 0.f;
@@ -975,10 +984,11 @@ static int eval_locked(bv_handle *h, const double *theta, double *llk)
         if (rc) return rc;
     }
     BV_CUDA_TRY(cudaEventRecord(h->ev0, h->stream));
-    if (h->gexec) {
-        BV_CUDA_TRY(cudaGraphLaunch(h->gexec, h->stream));
+    const int kind = eval_kind(h);
+    if (h->gexec[kind]) {
+        BV_CUDA_TRY(cudaGraphLaunch(h->gexec[kind], h->stream));
     } else {
-        rc = enqueue_eval(h, h->stream);
+        rc = enqueue_eval(h, h->stream, kind);
         if (rc) return rc;
     }
     BV_CUDA_TRY(cudaEventRecord(h->ev1, h->stream));
@@ -1008,8 +1018,10 @@ static int eval_locked(bv_handle *h, const double *theta, double *llk)
     // Without the FP32 pass every block takes the FP64 pass, on the streamed
     // kernel when it covers the layout.
     s.streamed_blocks = !mixed ? h->streamed_blocks : (!h->mixed.fp32 && h->mixed_lean ? h->owned : 0);
-    s.streamed_threads = s.streamed_blocks > 0 ? h->lean_threads : 0;
-    s.streamed_variant = s.streamed_blocks > 0 ? h->lean_vi : -1;
+    // The streamed launch is the last one planned.
+    const bv_handle::Kernel *lk = s.streamed_blocks > 0 ? &h->launches.back().k[kind] : nullptr;
+    s.streamed_threads = lk ? lk->threads : 0;
+    s.streamed_variant = lk ? lk->variant : -1;
     for (int i = 0; i < kNumLean; ++i) s.tune_ms[i] = h->tune_ms[i];
     s.llk = r.llk;
     s.device_ms = ms;

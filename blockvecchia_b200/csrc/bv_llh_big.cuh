@@ -30,13 +30,8 @@
 // Every wait on an mbarrier is bounded; a wait that gives up flags the block
 // BV_ST_DEVICE_TIMEOUT and the remaining waits are skipped.
 //
-// The same function with NS = 0 is the default path for every block whose
-// two panels fit (the multi-CTA streamed kernels llh_lean_kernel_t and
-// llh_lean_server_kernel, 96-256 threads, several CTAs per SM): no staging;
-// the update warps read the earlier panels' fragments straight from the slab
-// into registers and accumulate panel p+1's tiles in place on the DMMA
-// accumulators (panel_update_direct); optionally the whole matrix is
-// generated into the slab first (kBulk).
+// The default path for every block whose two panels fit (bv_llh_lean.cuh)
+// shares the slab and shared-memory layout and the panel structure.
 #pragma once
 
 #include <stdint.h>
@@ -129,21 +124,6 @@ inline size_t big_slab_stride(int max_m, int small_m, int big_m, int nz = 0)
 }
 
 __device__ __forceinline__ int swz(int r, int c) { return c ^ ((r & 3) << 2); }
-
-// CTA size of the multi-CTA streamed kernel for a launch whose largest block
-// has M = max_m, from the measured table (the handles and the server use
-// it): 128 threads x 4 CTAs per SM for small blocks, 160 x 3, 256 x 2.
-inline int lean_table_threads(int max_m) { return max_m <= 170 ? 128 : (max_m <= 250 ? 160 : 256); }
-
-// The static shared scratch the streamed path needs (a subset of
-// BlockShared), for kernels that run only this path.
-struct alignas(16) LeanShared {
-    double Lt[kNB][kNB];  // factored diagonal block, transposed
-    double inv[kNB];      // 1 / L_jj (0: failed pivot)
-    double red[2][kWarps];
-    unsigned status;
-    int task;
-};
 
 // Named barrier over warps 1..NT/32-1 (the update warps).
 template <int NT>
@@ -247,149 +227,22 @@ __device__ __forceinline__ void panel_update_tiles(double *dst, int dst_r0, cons
     }
 }
 
-// The left-looking update of panel p+1 without staging: nxt rows [n0, Mp)
-// (local row = i - n0) take panels q = 0..p-1 read straight from this CTA's
-// slab (L2).  Warps [w0, w0 + nw) own 8-row tiles (tile t on warp t mod nw)
-// and keep kDT of them in registers across all q, so the warps never wait
-// for one another; the next panel's fragments are loaded while the current
-// one is applied.  The tiles are the DMMA accumulators themselves: with B
-// negated, D = (-B)^T A + D subtracts each panel's products in place, 2 kDT
-// independent accumulation chains per warp.  Per element the operations and
-// their order do not depend on the CTA size or the tile count.  A lane's
-// DMMA steps 2h and 2h+1 use the adjacent columns k = 8h + 2 c4 + {0, 1},
-// one 16-byte load for both (the same columns in A and B, so each step
-// still sums four k-products).  kDT = 2 measured fastest (n = 1M, cs = 200:
-// 59.1 ms at 2, 63.4 at 3, 69.9 at 4; with 3 or more the live fragments
-// crowd the registers).
-constexpr int kDT = 2;
-
-// Substitution rows of the factor warp per panel (process_block_big): with
-// up to 256 rows below the diagonal block (every panel of M <= ~290) warp 0
-// solves them all while the other warps generate and update the next panel.
-// Kernel ms for n = 1M, cs = 200 / n = 200k, cs = 120 / n = 20k, cs = 300:
-// 32 rows 51.0 / 3.89 / 1.91, 64 rows 50.4 / 3.87 / 1.89, 128 rows 49.7 /
-// 3.78 / 1.86, 256 rows 49.2 / 3.77 / 1.84 (rows dealt over the whole CTA
-// after a barrier: 51.2 / 3.84 / 1.92).
+// Substitution rows of the factor warp per panel: with up to 256 rows below
+// the diagonal block (every panel of M <= ~290) warp 0 solves them all while
+// the other warps generate and update the next panel.  Kernel ms for n = 1M,
+// cs = 200 / n = 200k, cs = 120 / n = 20k, cs = 300: 32 rows 51.0 / 3.89 /
+// 1.91, 64 rows 50.4 / 3.87 / 1.89, 128 rows 49.7 / 3.78 / 1.86, 256 rows
+// 49.2 / 3.77 / 1.84 (rows dealt over the whole CTA after a barrier: 51.2 /
+// 3.84 / 1.92).
 constexpr int kSubstRows0 = 256;
-
-__device__ __forceinline__ double2 ldcg2(const double *p)
-{
-    return __ldcg(reinterpret_cast<const double2 *>(p));
-}
-
-template <int NTILE>
-__device__ __forceinline__ void load_frags(const double *pq, int q0, int Mp, int n0, int i0, int nw,
-                                           int r8, int c4, double2 (&bf)[2][2], double2 (&af)[NTILE][2])
-{
-    // B: the 16 rows n0.. of panel q, read by every tile of the panel,
-    // through L1 (n = 1M, cs = 200: 51.2 against 51.8 ms through L2 only);
-    // A: each tile's own rows, read once per panel, L2 only.  This CTA wrote
-    // both before the last barrier, from this SM.
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-#pragma unroll
-        for (int nj = 0; nj < 2; ++nj) {
-            const int r = n0 + 8 * nj + r8;
-            bf[h][nj] = (r < Mp) ? *reinterpret_cast<const double2 *>(pq + (size_t)(r - q0) * 16 +
-                                                                      swz(r, 8 * h + 2 * c4))
-                                 : make_double2(0.0, 0.0);
-        }
-#pragma unroll
-        for (int m = 0; m < NTILE; ++m) {
-            const int ia = i0 + 8 * nw * m + r8;
-            af[m][h] = (ia < Mp) ? ldcg2(pq + (size_t)(ia - q0) * 16 + swz(ia, 8 * h + 2 * c4))
-                                 : make_double2(0.0, 0.0);
-        }
-    }
-}
-
-template <int NTILE, bool kRaw>
-__device__ __forceinline__ void direct_tiles(double *nxt, int n0, const double *slab, int Mp, int p,
-                                             int i0, int nw, int r8, int c4)
-{
-    // Panel p+1 before the update: generated into nxt, or (kRaw) still in
-    // the slab where the whole matrix was generated.
-    const double *src = kRaw ? slab + big_panel_base(p + 1, Mp) : nxt;
-    double d[NTILE][2][2];
-#pragma unroll
-    for (int m = 0; m < NTILE; ++m) {
-        const int ia = i0 + 8 * nw * m + r8;
-#pragma unroll
-        for (int nj = 0; nj < 2; ++nj)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int o = (ia - n0) * 16 + swz(ia, 8 * nj + 2 * c4 + e);
-                d[m][nj][e] = (ia < Mp) ? (kRaw ? __ldcg(src + o) : src[o]) : 0.0;
-            }
-    }
-    double2 bf[2][2], af[NTILE][2], bn[2][2], an[NTILE][2];
-    if (p > 0) load_frags<NTILE>(slab + big_panel_base(0, Mp), 0, Mp, n0, i0, nw, r8, c4, bf, af);
-    for (int q = 0; q < p; ++q) {
-        if (q + 1 < p)
-            load_frags<NTILE>(slab + big_panel_base(q + 1, Mp), (q + 1) * kNB, Mp, n0, i0, nw, r8, c4,
-                              bn, an);
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-            const int h = kk >> 1;
-            double b[2];
-#pragma unroll
-            for (int nj = 0; nj < 2; ++nj) b[nj] = -((kk & 1) ? bf[h][nj].y : bf[h][nj].x);
-#pragma unroll
-            for (int m = 0; m < NTILE; ++m) {
-                const double a = (kk & 1) ? af[m][h].y : af[m][h].x;
-#pragma unroll
-                for (int nj = 0; nj < 2; ++nj) dmma_8x8x4(d[m][nj][0], d[m][nj][1], a, b[nj]);
-            }
-        }
-        if (q + 1 < p) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-#pragma unroll
-                for (int nj = 0; nj < 2; ++nj) bf[h][nj] = bn[h][nj];
-#pragma unroll
-                for (int m = 0; m < NTILE; ++m) af[m][h] = an[m][h];
-            }
-        }
-    }
-#pragma unroll
-    for (int m = 0; m < NTILE; ++m) {
-        const int ia = i0 + 8 * nw * m + r8;
-        if (ia < Mp) {
-#pragma unroll
-            for (int nj = 0; nj < 2; ++nj)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) nxt[(ia - n0) * 16 + swz(ia, 8 * nj + 2 * c4 + e)] = d[m][nj][e];
-        }
-    }
-}
-
-// kRaw: panel p+1 is taken from the slab (the whole matrix generated there
-// first) and written to nxt updated, also when there is nothing to apply.
-template <bool kRaw>
-__device__ __forceinline__ void panel_update_direct(double *nxt, int n0, const double *slab, int Mp, int p,
-                                                    int w0, int nw)
-{
-    const int warp = (threadIdx.x >> 5) - w0, lane = threadIdx.x & 31;
-    if (warp < 0 || warp >= nw || (!kRaw && p == 0)) return;
-    const int r8 = lane >> 2, c4 = lane & 3;
-    const int ntiles = (Mp - n0 + 7) >> 3;
-    // Groups of kDT tiles per warp, computed whole: the tiles of a group
-    // beyond the panel's rows hold zeros and are not stored (one code path
-    // keeps the accumulation chains of all kDT tiles interleaved).
-    for (int t0 = warp; t0 < ntiles; t0 += nw * kDT)
-        direct_tiles<kDT, kRaw>(nxt, n0, slab, Mp, p, n0 + 8 * t0, nw, r8, c4);
-}
 
 // One block by the streamed path, run by a CTA of NT threads (warp 0
 // factors, the other NT/32 - 1 warps generate and update), with RC rows per
-// streamed chunk and NS chunks in flight (NS = 0: no staging, the warps read
-// the slab directly, panel_update_direct; with kBulk the whole matrix is
-// generated into the slab first).  smem: the dynamic area
+// streamed chunk and NS chunks in flight.  smem: the dynamic area
 // (big_layout(M, RC, nz, NS).total bytes); slab: this CTA's global slab
 // (big_slab_doubles(M) doubles).  Every element's operations and their
-// order are the same for every NT, RC, NS > 0 and kBulk; the direct update
-// (NS = 0) accumulates in place and rounds differently from the staged one.
-template <int NT, int RC, typename SH, int NS = kBigStages, bool kXYZ3 = false, bool kBulk = false>
+// order are the same for every NT, RC and NS.
+template <int NT, int RC, typename SH, int NS = kBigStages, bool kXYZ3 = false>
 static __device__ __noinline__ void process_block_big(const LlhArgs &a, const MaternParams &mp, int b,
                                                       unsigned char *smem, double *slab, SH &sh)
 {
@@ -408,7 +261,7 @@ static __device__ __noinline__ void process_block_big(const LlhArgs &a, const Ma
     double *T = kXYZ3 ? reinterpret_cast<double *>(smem + l.o_T) : nullptr;
     double *cur = reinterpret_cast<double *>(smem + l.o_cur);
     double *nxt = reinterpret_cast<double *>(smem + l.o_next);
-    double *stage[NS > 0 ? NS : 1];
+    double *stage[NS];
 #pragma unroll
     for (int st = 0; st < NS; ++st) stage[st] = reinterpret_cast<double *>(smem + l.o_stage[st]);
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem + l.o_bar);
@@ -426,20 +279,8 @@ static __device__ __noinline__ void process_block_big(const LlhArgs &a, const Ma
         fence_mbar_init();
     }
     __syncthreads();
-    if constexpr (NS == 0 && kBulk) {
-        // Every panel's entries straight into the slab, by all warps (the
-        // update warps then take panel p+1 from there): the generation runs
-        // at the CTA's full width instead of beside warp 0's pivot chain.
-        for (int q = 0; q < P; ++q)
-            gen_column<kXYZ3>(slab + big_panel_base(q, Mp), q * kNB, X, Y, Z, T, M, Mp, q * kNB,
-                              min(kNB, M - q * kNB), tid & 15, q * kNB + (tid >> 4), kT >> 4, mp);
-        __syncthreads();
-        for (int e = tid; e < Mp * 8; e += kT)
-            reinterpret_cast<double2 *>(cur)[e] = __ldcg(reinterpret_cast<const double2 *>(slab) + e);
-    } else {
-        // Panel 0 into cur: thread t takes column t mod 16, every (kT/16)-th row.
-        gen_column<kXYZ3>(cur, 0, X, Y, Z, T, M, Mp, 0, min(kNB, M), tid & 15, tid >> 4, kT >> 4, mp);
-    }
+    // Panel 0 into cur: thread t takes column t mod 16, every (kT/16)-th row.
+    gen_column<kXYZ3>(cur, 0, X, Y, Z, T, M, Mp, 0, min(kNB, M), tid & 15, tid >> 4, kT >> 4, mp);
     __syncthreads();
 
     unsigned st = 0;          // thread 0: pivot flags
@@ -476,17 +317,12 @@ static __device__ __noinline__ void process_block_big(const LlhArgs &a, const Ma
             if (lane == 0) st |= fst;
         } else if (kb1 > 0) {
             const int nrows = Mp - n0;
-            if constexpr (NS != 0 || !kBulk) {
-                // Panel p+1: generate (update thread u takes column u mod 16,
-                // every ((kT - 32)/16)-th row), then apply panels 0..p-1.
-                const int u = tid - 32;
-                gen_column<kXYZ3>(nxt, n0, X, Y, Z, T, M, Mp, n0, kb1, u & 15, n0 + (u >> 4), (kT - 32) >> 4,
-                                  mp);
-                update_warps_sync<NT>();
-            }
-            if constexpr (NS == 0) {
-                panel_update_direct<kBulk>(nxt, n0, slab, Mp, p, 1, kW - 1);
-            } else {
+            // Panel p+1: generate (update thread u takes column u mod 16,
+            // every ((kT - 32)/16)-th row), then apply panels 0..p-1.
+            const int u = tid - 32;
+            gen_column<kXYZ3>(nxt, n0, X, Y, Z, T, M, Mp, n0, kb1, u & 15, n0 + (u >> 4), (kT - 32) >> 4,
+                              mp);
+            update_warps_sync<NT>();
             const int nchunk = (nrows + RC - 1) / RC;
             const int items = nchunk * p;       // (chunk, q), q fastest
             const bool producer = (tid == 32);
@@ -539,7 +375,6 @@ static __device__ __noinline__ void process_block_big(const LlhArgs &a, const Ma
                 // is used again: wait (bounded) for each stage's last phase.
                 for (int s = 0; s < NS; ++s)
                     if (issued[s] > landed[s]) mbar_wait_bounded(&bar[s], (unsigned)(issued[s] - 1) & 1u);
-            }
             }
         }
         // The substitution needs only the factored diagonal block: warp 0

@@ -1,0 +1,656 @@
+// bv_llh_lean.cuh -- the default FP64 block evaluation: the left-looking
+// blocked Cholesky of bv_llh_big.cuh (same augmented system, panels, slab and
+// shared-memory layout) run by small CTAs of 96-256 threads, several per SM,
+// so that the pivot chains of several blocks overlap on one SM.
+//
+// Per 16-column panel p, warp 0 factors panel p's diagonal block and solves
+// the rows below it while the other warps bring panel p+1 up to date.  An
+// update warp owns groups of kDT tiles of 8 rows x 16 columns of panel p+1
+// and keeps a group's entries in the DMMA accumulators from their generation
+// to their last update from the slab:
+//   * the lane that holds entry (i, j) in the m8n8k4 accumulator layout
+//     evaluates its covariance (4 kDT independent entries per lane, so the
+//     square-root and exponential chains overlap) -- the panel never makes
+//     the round trip through shared memory between generation and update;
+//   * panels 0..p-1 are applied straight from the CTA's slab (L2-resident),
+//     the next panel's fragments loaded while the current one is applied.
+//     The accumulators hold the entries negated, so D = A B + D subtracts
+//     each product in place without negating an operand; rounding is
+//     symmetric, so the bits are those of x - a b.
+// Then panel p goes to the slab and panel p+1 takes panel p's update from
+// shared memory.
+//
+// Per element the operations and their order do not depend on the CTA size,
+// the tile count or where the entry was generated, so every variant gives
+// the same bits.
+#pragma once
+
+#include "bv_llh_big.cuh"
+
+namespace bv {
+
+// How a block's entries are generated: the closed forms on 2-D locations in
+// the update warps' accumulators; a general nu (K_nu) and locations with a
+// third coordinate (cov_xyz), which are long, through shared memory.  Each is
+// a kernel of its own: with the long ones beside it (inlined or called) the
+// closed forms' kernel spills 500-900 bytes per thread (n = 1M, cs = 200: 55
+// against 44 ms).
+enum LeanGen : int { kGenClosed = 0, kGenGeneral = 1, kGenXYZ = 2 };
+
+// CTA size of the streamed kernel for a launch of `blocks` blocks, the largest
+// of M = max_m (the handles and the server use it).  Multiples of 128 threads
+// keep warp 0, whose pivot chain is the block's critical path, on an SM
+// sub-partition without update warps: a warp issuing FP64 MMAs back to back
+// beside the chain stretched it from 5.2k to 16.9k cycles per panel.  Below M ~
+// 115 the panels leave an update warp too few tiles, and 96 threads with four
+// CTAs per SM win; beyond M ~ 240 only two CTAs' panels fit an SM, and 256
+// threads give them as many update warps as registers allow.  A launch that
+// leaves SMs with one or two blocks wants each block short: 128 threads.
+// Entries generated through shared memory are a larger share of the update
+// warps' work: more of them.  Kernel ms at 96 x 4 CTAs per SM / 160 x 3 /
+// 256 x 2 / 128 x 3 / 160 x 2:
+//   cs =  30, classic, 30k blocks (M <=  31): 0.55 / 0.94 / 1.30 / 0.66 / 0.96
+//   cs =  60, 150 blocks (M <=  82):          .042 / .047 / .045 / .036 / .037
+//   cs =  60, 5k blocks (M <=  77):           0.27 / 0.42 / 0.55 / 0.30 / 0.39
+//   cs =  80, 10k blocks (M <=  97):          0.77 / 1.13 / 1.44 / 0.80 / 1.01
+//   cs = 120, 20k blocks (M <= 137):          3.15 / 3.88 / 4.63 / 2.96 / 3.48
+//   cs = 160, 10k blocks (M <= 177):          2.74 / 3.20 / 3.40 / 2.66 / 2.85
+//   cs = 200, 100k blocks (M <= 217):         53.1 / 50.9 / 48.8 / 44.0 / 45.5
+//   cs = 240, 10k blocks (M <= 257):          7.29 / 6.96 / 6.68 / 6.19 / 6.09
+//   cs = 300, 1.5k blocks (M <= 322):         2.69 / 1.93 / 1.73 / 1.96 / 1.76
+//   space-time, cs = 100, 2.5k (M <= 114):    1.26 / 1.00 / 0.99 / 1.13 / 1.28
+//   nu = 0.8, cs = 120, 10k (M <= 137):       7.86 / 6.46 / 5.92 / 7.19 / 7.56
+inline int lean_table_threads(int gen, int max_m, size_t blocks)
+{
+    if (max_m > 250 || gen != kGenClosed) return 256;
+    return (max_m <= 115 && blocks > 600) ? 96 : 128;
+}
+
+// The static shared scratch the streamed path needs (a subset of
+// BlockShared), for kernels that run only this path.
+struct alignas(16) LeanShared {
+    double Lt[kNB][kNB];  // factored diagonal block, transposed
+    double inv[kNB];      // 1 / L_jj (0: failed pivot)
+    double ex[4][8];      // factor_panel's exchange of a 4 x 4 diagonal block
+    double red[2][8];     // per-warp sums (at most 8 warps)
+    unsigned status;
+    int task;
+};
+
+// Tiles of a group.  Two measured fastest (n = 1M, cs = 200: 59.1 ms at 2,
+// 63.4 at 3, 69.9 at 4 with the entries generated in shared memory: with 3 or
+// more the live fragments crowd the registers).
+constexpr int kDT = 2;
+
+__device__ __forceinline__ double2 ldcg2(const double *p)
+{
+    return __ldcg(reinterpret_cast<const double2 *>(p));
+}
+
+__device__ __forceinline__ double2 ld2(const double *p) { return *reinterpret_cast<const double2 *>(p); }
+
+// A lane's place in an 8-row tile (DMMA m8n8k4: row l >> 2, column pair
+// 2 (l & 3)).  Tiles start at multiples of 8 rows, so the slab swizzle is a
+// constant of the lane: columns 2 c4, 2 c4 + 1 at o0, 8 + 2 c4, + 1 at o1.
+struct TileLane {
+    int r8, c4, o0, o1;
+    __device__ __forceinline__ TileLane()
+    {
+        const int lane = threadIdx.x & 31;
+        r8 = lane >> 2;
+        c4 = lane & 3;
+        o0 = swz(r8, 2 * c4);
+        o1 = swz(r8, 8 + 2 * c4);
+    }
+};
+
+// Entries of NTILE tiles of the panel starting at row and column n0, negated:
+// tile m's rows i0 + m * rstep + r8, columns n0 + 8 nj + 2 c4 + e.  Rows
+// beyond the block and entries above the diagonal are zeros; row M holds the
+// observations; columns beyond the block are unspecified (never used).  The
+// values are those of big_entry for the closed forms (nu = 1/2, 3/2, 5/2),
+// which share the distance and the exponential; the 4 NTILE entries of a lane
+// are independent chains.
+template <int NTILE>
+__device__ __forceinline__ void gen_tiles(double (&d)[NTILE][2][2], const double *X, const double *Y,
+                                          const double *Z, int M, int n0, int i0, int rstep,
+                                          const TileLane &L, const MaternParams *mp)
+{
+    const int kind = __ldg(&mp->nu_kind);
+    const double range = __ldg(&mp->range), inv_range = __ldg(&mp->inv_range);
+    double xj[4], yj[4];
+#pragma unroll
+    for (int nj = 0; nj < 2; ++nj) {
+        const double2 a = ld2(X + n0 + 8 * nj + 2 * L.c4), b = ld2(Y + n0 + 8 * nj + 2 * L.c4);
+        xj[2 * nj] = a.x;
+        xj[2 * nj + 1] = a.y;
+        yj[2 * nj] = b.x;
+        yj[2 * nj + 1] = b.y;
+    }
+    double r[NTILE][4];
+#pragma unroll
+    for (int m = 0; m < NTILE; ++m) {
+        const int i = min(i0 + m * rstep + L.r8, M - 1);
+        const double xi = X[i], yi = Y[i];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const double dx = xj[c] - xi, dy = yj[c] - yi;
+            r[m][c] = div_by_recip(__dsqrt_rn(__fma_rn(dx, dx, __dmul_rn(dy, dy))), range, inv_range);
+        }
+    }
+    if (!__ldg(&mp->scale_is_one)) {
+        const double ds = __ldg(&mp->dist_scale), inv_ds = __ldg(&mp->inv_ds);
+#pragma unroll
+        for (int m = 0; m < NTILE; ++m)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) r[m][c] = div_by_recip(r[m][c], ds, inv_ds);
+    }
+    const double sigma2 = __ldg(&mp->sigma2);
+#pragma unroll
+    for (int m = 0; m < NTILE; ++m)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const double e = exp(-r[m][c]);
+            d[m][c >> 1][c & 1] = e;
+        }
+    if (kind == kNuThreeHalves) {
+#pragma unroll
+        for (int m = 0; m < NTILE; ++m)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) d[m][c >> 1][c & 1] *= __dadd_rn(1.0, r[m][c]);
+    } else if (kind == kNuFiveHalves) {
+#pragma unroll
+        for (int m = 0; m < NTILE; ++m)
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                d[m][c >> 1][c & 1] *=
+                    __fma_rn(r[m][c], __dmul_rn(r[m][c], 1.0 / 3.0), __dadd_rn(1.0, r[m][c]));
+    }
+#pragma unroll
+    for (int m = 0; m < NTILE; ++m)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            double &v = d[m][c >> 1][c & 1];
+            v = (r[m][c] == 0.0) ? -sigma2 : __dmul_rn(-sigma2, v);
+        }
+    const double nugget = __ldg(&mp->nugget);
+#pragma unroll
+    for (int m = 0; m < NTILE; ++m) {
+        const int i = i0 + m * rstep + L.r8;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int j = n0 + 8 * (c >> 1) + 2 * L.c4 + (c & 1);
+            double &v = d[m][c >> 1][c & 1];
+            if (i >= M) v = (i == M) ? -Z[j] : 0.0;
+            else if (j >= i) v = (j == i) ? __dsub_rn(v, nugget) : 0.0;
+        }
+    }
+}
+
+// Fragments of one slab panel for a group of NTILE tiles: B, the 16 rows n0..
+// that every tile of the panel multiplies by, through L1 (n = 1M, cs = 200:
+// 51.2 against 51.8 ms through L2 only); A, each tile's own rows, read once
+// per panel, L2 only.  This CTA wrote both before the last barrier, from
+// this SM.  Rows beyond the block read the following panel's memory (panel
+// q + 1 holds at least 18 rows whenever panel q is applied); they only reach
+// rows and columns that are never stored or never used.
+template <int NTILE>
+struct Frags {
+    double2 b[2][2], a[NTILE][2];
+    __device__ __forceinline__ void load(const double *pb, const double *pa, int tstep, const TileLane &L)
+    {
+#pragma unroll
+        for (int nj = 0; nj < 2; ++nj) {
+            b[0][nj] = ld2(pb + 128 * nj + L.o0);
+            b[1][nj] = ld2(pb + 128 * nj + L.o1);
+        }
+#pragma unroll
+        for (int m = 0; m < NTILE; ++m) {
+            a[m][0] = ldcg2(pa + m * tstep + L.o0);
+            a[m][1] = ldcg2(pa + m * tstep + L.o1);
+        }
+    }
+    // A lane's DMMA steps 2h and 2h+1 use the adjacent columns k = 8h + 2 c4
+    // + {0, 1}, one 16-byte load for both.
+    __device__ __forceinline__ void apply(double (&d)[NTILE][2][2]) const
+    {
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+            for (int m = 0; m < NTILE; ++m)
+#pragma unroll
+                for (int nj = 0; nj < 2; ++nj)
+                    dmma_8x8x4(d[m][nj][0], d[m][nj][1], (kk & 1) ? a[m][kk >> 1].y : a[m][kk >> 1].x,
+                               (kk & 1) ? b[kk >> 1][nj].y : b[kk >> 1][nj].x);
+    }
+};
+
+// NTILE tiles (first tile at row i0, the others rstep rows further each) take
+// panels 0..p-1 from the slab.  Row i of panel q is at slab + 16 (q (Mp - 8q
+// - 8) + i).
+template <int NTILE>
+__device__ __forceinline__ void update_tiles(double (&d)[NTILE][2][2], const double *slab, int Mp, int p,
+                                             int n0, int i0, int rstep, const TileLane &L)
+{
+    if (p == 0) return;
+    const double *pb = slab + 16 * (n0 + L.r8), *pa = slab + 16 * (i0 + L.r8);
+    const int tstep = 16 * rstep;
+    int step = 16 * (Mp - 16);  // from panel q to q + 1
+    Frags<NTILE> f0, f1;
+    f0.load(pb, pa, tstep, L);
+    for (int q = 0; q < p; q += 2) {
+        if (q + 1 < p) {
+            pb += step;
+            pa += step;
+            step -= 256;
+            f1.load(pb, pa, tstep, L);
+        }
+        f0.apply(d);
+        if (q + 1 < p) {
+            if (q + 2 < p) {
+                pb += step;
+                pa += step;
+                step -= 256;
+                f0.load(pb, pa, tstep, L);
+            }
+            f1.apply(d);
+        }
+    }
+}
+
+// Panel p+1 (rows n0..): its tiles evaluated by the lanes that hold them
+// (kGen) or read from the shared panel (generated there, positive), panels
+// 0..p-1 applied, the negated entries into nxt.  Warps [w0, w0 + nw) take
+// tiles t, t + nw, ...
+template <int NTILE, bool kGen>
+__device__ __forceinline__ void next_tiles(double *nxt, const double *X, const double *Y, const double *Z,
+                                           const double *slab, int M, int p, int n0, int t0, int nw,
+                                           const TileLane &L, const MaternParams *mp)
+{
+    const int Mp = M + 1, i0 = n0 + 8 * t0, rstep = 8 * nw;
+    double d[NTILE][2][2];
+    if constexpr (kGen) {
+        gen_tiles<NTILE>(d, X, Y, Z, M, n0, i0, rstep, L, mp);
+    } else {
+#pragma unroll
+        for (int m = 0; m < NTILE; ++m) {
+            const double *row = nxt + 16 * (min(i0 + m * rstep + L.r8, M) - n0);
+#pragma unroll
+            for (int nj = 0; nj < 2; ++nj) {
+                const double2 v = ld2(row + (nj ? L.o1 : L.o0));
+                d[m][nj][0] = -v.x;
+                d[m][nj][1] = -v.y;
+            }
+        }
+    }
+    update_tiles<NTILE>(d, slab, Mp, p, n0, i0, rstep, L);
+#pragma unroll
+    for (int m = 0; m < NTILE; ++m) {
+        const int i = i0 + m * rstep + L.r8;
+        if (i < Mp) {
+            double *row = nxt + 16 * (i - n0);
+            *reinterpret_cast<double2 *>(row + L.o0) = make_double2(d[m][0][0], d[m][0][1]);
+            *reinterpret_cast<double2 *>(row + L.o1) = make_double2(d[m][1][0], d[m][1][1]);
+        }
+    }
+}
+
+template <bool kGen>
+__device__ __forceinline__ void next_panel(double *nxt, const double *X, const double *Y, const double *Z,
+                                           const double *slab, int M, int p, int n0, int w0, int nw,
+                                           const MaternParams *mp)
+{
+    const TileLane L;
+    const int ntiles = (M + 8 - n0) >> 3;  // rows n0..M
+    for (int t0 = (threadIdx.x >> 5) - w0; t0 < ntiles; t0 += nw * kDT) {
+        if (t0 + nw < ntiles)
+            next_tiles<kDT, kGen>(nxt, X, Y, Z, slab, M, p, n0, t0, nw, L, mp);
+        else
+            next_tiles<1, kGen>(nxt, X, Y, Z, slab, M, p, n0, t0, nw, L, mp);
+    }
+}
+
+// Panel p+1 (negated in nxt, rows n0..M) takes panel p's update from cur
+// (rows k0.., panel p's B rows n0..n0+15): the products are summed from zero
+// and subtracted, entries back to their own sign.  Tiles dealt to all warps.
+template <int NT>
+__device__ __forceinline__ void last_update(double *nxt, const double *cur, int M, int k0, int n0)
+{
+    const TileLane L;
+    const int x = (L.r8 & 3) << 2;
+    const double *brow = cur + 16 * (n0 - k0 + L.r8) + L.c4;
+    double b[4][2];
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+        for (int nj = 0; nj < 2; ++nj)
+            b[kk][nj] = (n0 + 8 * nj + L.r8 <= M) ? brow[128 * nj + ((4 * kk) ^ x)] : 0.0;
+    for (int i0 = n0 + 8 * (threadIdx.x >> 5); i0 <= M; i0 += NT / 4) {
+        const int i = i0 + L.r8;
+        const bool in = i <= M;
+        const double *arow = cur + 16 * (min(i, M) - k0) + L.c4;
+        double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+            const double a = arow[(4 * kk) ^ x];
+#pragma unroll
+            for (int nj = 0; nj < 2; ++nj) dmma_8x8x4(acc[nj][0], acc[nj][1], a, b[kk][nj]);
+        }
+        if (in) {
+            double2 *d0 = reinterpret_cast<double2 *>(nxt + 16 * (i - n0) + L.o0);
+            double2 *d1 = reinterpret_cast<double2 *>(nxt + 16 * (i - n0) + L.o1);
+            const double2 v0 = *d0, v1 = *d1;
+            *d0 = make_double2(-v0.x - acc[0][0], -v0.y - acc[0][1]);
+            *d1 = make_double2(-v1.x - acc[1][0], -v1.y - acc[1][1]);
+        }
+    }
+}
+
+// A row of 16 swizzled doubles (absolute row r) to and from registers.
+__device__ __forceinline__ void load_row(const double *row, int r, double (&v)[kNB])
+{
+    const int x = (r & 3) << 2;
+#pragma unroll
+    for (int h = 0; h < kNB / 2; ++h) {
+        const double2 t = ld2(row + ((2 * h) ^ x));
+        v[2 * h] = t.x;
+        v[2 * h + 1] = t.y;
+    }
+}
+
+__device__ __forceinline__ void store_row(double *row, int r, const double (&v)[kNB])
+{
+    const int x = (r & 3) << 2;
+#pragma unroll
+    for (int h = 0; h < kNB / 2; ++h)
+        *reinterpret_cast<double2 *>(row + ((2 * h) ^ x)) = make_double2(v[2 * h], v[2 * h + 1]);
+}
+
+// The diagonal block of panel p (rows k0.., kb <= 16 columns) and the 16 rows
+// below it, by one warp: lane r holds row k0 + r in v (zeros above the
+// diagonal and beyond the block).  The element operations and their order are
+// factor_rows' (lagged Crout: the products over k < c - 1 in four partial
+// sums by k mod 4, the k = c - 1 product last).
+//
+// The warp's time is the dependent chain of 16 pivots (an FP64 rsqrt is ~60
+// cycles, a shuffle 26 and more when the SM's shared-memory pipe is busy), so
+// four columns are done per round: the lanes' partial sums over the earlier
+// columns are formed by themselves, the 4 x 4 diagonal block's go to every
+// lane through `ex`, and every lane factors that block redundantly and
+// applies it to its own row -- two shared-memory exchanges per four pivots
+// instead of eight to thirty-two shuffles per pivot, no divergent branches.
+// Alone on an SM sub-partition: 4.6k cycles per panel with shuffles and a
+// guard per pivot, 3.5k this way, and fewer shared-memory operations for the
+// other CTAs' warps to queue behind.
+//
+// Lt receives the factor transposed (zeros above the diagonal and in columns
+// beyond kb); myinv is 1 / L_rr of a lane's own pivot (0: failed).
+__device__ __forceinline__ unsigned factor_panel(int k0, int kb, int mc, double (&v)[kNB], double &myinv,
+                                                 double (*Lt)[kNB], double (*ex)[8])
+{
+    const int lane = threadIdx.x & 31;
+    const bool low = lane < kNB;
+    unsigned st = 0;
+    myinv = 0.0;
+#pragma unroll
+    for (int c0 = 0; c0 < kNB; c0 += 4) {
+        // Columns c0, c0+1: complete sums but for the products of this round;
+        // c0+2, c0+3: partial sums 0, 1 and the sum of 2 and 3.
+        double s0, s1, g2[3], g3[3];
+        if (c0 == 0) {
+            s0 = v[0];
+            s1 = v[1];
+            g2[0] = v[2];
+            g3[0] = v[3];
+            g2[1] = g2[2] = g3[1] = g3[2] = 0.0;
+        } else {
+            double a[4][4], last = 0.0;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                a[c][0] = v[c0 + c];
+                a[c][1] = a[c][2] = a[c][3] = 0.0;
+            }
+#pragma unroll
+            for (int k = 0; k < c0; ++k) {
+                // Four columns' loads at a time (more would spill).
+                if ((k & 3) == 0) asm volatile("" ::: "memory");
+                const double2 x = ld2(&Lt[k][c0]), y = ld2(&Lt[k][c0 + 2]);
+                if (k == c0 - 1)
+                    last = x.x;
+                else
+                    a[0][k & 3] = fma(-v[k], x.x, a[0][k & 3]);
+                a[1][k & 3] = fma(-v[k], x.y, a[1][k & 3]);
+                a[2][k & 3] = fma(-v[k], y.x, a[2][k & 3]);
+                a[3][k & 3] = fma(-v[k], y.y, a[3][k & 3]);
+            }
+            s0 = fma(-v[c0 - 1], last, (a[0][0] + a[0][1]) + (a[0][2] + a[0][3]));
+            s1 = (a[1][0] + a[1][1]) + (a[1][2] + a[1][3]);
+            g2[0] = a[2][0];
+            g2[1] = a[2][1];
+            g2[2] = a[2][2] + a[2][3];
+            g3[0] = a[3][0];
+            g3[1] = a[3][1];
+            g3[2] = a[3][2] + a[3][3];
+        }
+        if (lane >= c0 && lane < c0 + 4) {
+            double2 *e = reinterpret_cast<double2 *>(ex[lane - c0]);
+            e[0] = make_double2(s0, s1);
+            e[1] = make_double2(g2[0], g2[1]);
+            e[2] = make_double2(g2[2], g3[0]);
+            e[3] = make_double2(g3[1], g3[2]);
+        }
+        __syncwarp();
+        const double2 e1 = ld2(&ex[1][0]);
+        const double2 e2a = ld2(&ex[2][0]), e2b = ld2(&ex[2][2]);
+        const double2 e3a = ld2(&ex[3][0]), e3b = ld2(&ex[3][2]), e3c = ld2(&ex[3][4]), e3d = ld2(&ex[3][6]);
+        const double e0 = ex[0][0], e2c = ex[2][4];
+        double piv[4], inv[4], w[4];
+        bool ok[4];
+        // A failed pivot's column is zero below it; rsqrt of 1 keeps the
+        // evaluation branch-free.
+        auto pivot = [&](int c, double x) {
+            piv[c] = x;
+            ok[c] = x > 0.0;
+            const double y = rsqrt(ok[c] ? x : 1.0);
+            inv[c] = ok[c] ? y : 0.0;
+        };
+        pivot(0, e0);
+        const double l10 = e1.x * inv[0], l20 = e2a.x * inv[0], l30 = e3a.x * inv[0];
+        w[0] = s0 * inv[0];
+        pivot(1, fma(-l10, l10, e1.y));
+        const double l21 = fma(-l20, l10, e2a.y) * inv[1], l31 = fma(-l30, l10, e3a.y) * inv[1];
+        w[1] = fma(-w[0], l10, s1) * inv[1];
+        pivot(2, fma(-l21, l21, (fma(-l20, l20, e2b.x) + e2b.y) + e2c));
+        const double l32 = fma(-l31, l21, (fma(-l30, l20, e3b.x) + e3b.y) + e3c.x) * inv[2];
+        w[2] = fma(-w[1], l21, (fma(-w[0], l20, g2[0]) + g2[1]) + g2[2]) * inv[2];
+        pivot(3, fma(-l32, l32, (fma(-l30, l30, e3c.y) + fma(-l31, l31, e3d.x)) + e3d.y));
+        w[3] = fma(-w[2], l32, (fma(-w[0], l30, g3[0]) + fma(-w[1], l31, g3[1])) + g3[2]) * inv[3];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int q = c0 + c;
+            if (!ok[c] && q < kb) st |= (k0 + q < mc) ? 1u : 2u;
+            const double dq = ok[c] ? piv[c] * inv[c] : piv[c];
+            v[q] = (lane > q) ? w[c] : ((lane == q) ? dq : v[q]);
+            if (lane == q) myinv = inv[c];
+            if (low) Lt[q][lane] = (lane < kb) ? v[q] : 0.0;
+        }
+        __syncwarp();
+    }
+    return st;
+}
+
+// The factor warp's part of panel p (rows k0.. in cur): lane r < kb owns row
+// k0+r of the diagonal block; with a full panel the upper lanes solve the
+// next 16 rows on the same chain, so the substitution starts 16 rows on.
+__device__ __forceinline__ unsigned factor_phase(double *cur, int M, int k0, int kb, int mc, LeanShared &sh)
+{
+    const int lane = threadIdx.x & 31;
+    const bool low = lane < kNB;
+    const int row = k0 + lane;
+    const bool valid = low ? lane < kb : (kb == kNB && row <= M);
+    double *rowp = cur + (valid ? lane : 0) * 16;
+    double v[kNB], myinv;
+    load_row(rowp, valid ? row : k0, v);
+#pragma unroll
+    for (int c = 0; c < kNB; ++c)
+        if (!(valid && c < kb && (!low || c <= lane))) v[c] = 0.0;
+    const unsigned st = factor_panel(k0, kb, mc, v, myinv, sh.Lt, sh.ex);
+    if (valid) store_row(rowp, row, v);
+    if (low) sh.inv[lane] = (lane < kb) ? myinv : 0.0;
+    return st;
+}
+
+// Row r below the diagonal block by forward substitution against L_kk.
+// Columns beyond a partial panel have zeros in Lt and inv.
+__device__ __forceinline__ void solve_row(const LeanShared &sh, double *row, int r)
+{
+    double w[kNB];
+    load_row(row, r, w);
+    double inv_q = sh.inv[0];
+    double l_next = sh.Lt[0][1];
+#pragma unroll
+    for (int q = 0; q < kNB; ++q) {
+        // The two operands on step q+1's dependent chain (1 / L_{q+1,q+1} and
+        // L_{q+2,q+1}) are read one step ahead; the fence keeps the others
+        // from being hoisted into spills.
+        asm volatile("" ::: "memory");
+        const double inv_cur = inv_q;
+        const double l_cur = l_next;
+        if (q + 1 < kNB) inv_q = sh.inv[q + 1];
+        if (q + 2 < kNB) l_next = sh.Lt[q + 1][q + 2];
+        double2 col[kNB / 2];
+#pragma unroll
+        for (int h = (q + 2) >> 1; h < kNB / 2; ++h) col[h] = ld2(&sh.Lt[q][2 * h]);
+        w[q] *= inv_cur;
+        if (q + 1 < kNB) w[q + 1] = fma(-w[q], l_cur, w[q + 1]);
+#pragma unroll
+        for (int c = q + 2; c < kNB; ++c) w[c] = fma(-w[q], (c & 1) ? col[c >> 1].y : col[c >> 1].x, w[c]);
+    }
+    store_row(row, r, w);
+}
+
+// One block by the streamed path, run by a CTA of NT threads (warp 0 factors
+// and solves, the other NT/32 - 1 warps generate and update).  smem: the
+// dynamic area (big_layout(M, 0, nz, 0).total bytes); slab: this CTA's global
+// slab (big_slab_doubles(M) doubles).
+template <int NT, int GEN>
+__device__ __forceinline__ void process_block_lean(const LlhArgs &a, const MaternParams *mp, int b,
+                                                          unsigned char *smem, double *slab, LeanShared &sh)
+{
+    static_assert(NT % 32 == 0 && NT > 32, "whole warps, at least one besides the factor warp");
+    constexpr bool kXYZ3 = GEN == kGenXYZ;
+    constexpr int kT = NT, kW = NT / 32;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int off = a.acc[b];
+    const int bs = a.acc[b + 1] - off;
+    const int mc = (b == 0) ? 0 : a.cs;
+    const int M = mc + bs, Mp = M + 1;
+    const int P = big_panels(M);
+    const BigLayout l = big_layout(M, 0, kXYZ3 ? 1 : 0, 0);
+    double *X = reinterpret_cast<double *>(smem + l.o_X);
+    double *Y = reinterpret_cast<double *>(smem + l.o_Y);
+    double *Z = reinterpret_cast<double *>(smem + l.o_Z);
+    double *T = kXYZ3 ? reinterpret_cast<double *>(smem + l.o_T) : nullptr;
+    double *cur = reinterpret_cast<double *>(smem + l.o_cur);
+    double *nxt = reinterpret_cast<double *>(smem + l.o_next);
+
+    const int *kidx = a.knn + (size_t)b * a.cs;
+    for (int t = tid; t < M; t += kT) {
+        const int src = (t < mc) ? __ldg(kidx + t) : off + (t - mc);
+        X[t] = __ldg(a.x + src);
+        Y[t] = __ldg(a.y + src);
+        Z[t] = __ldg(a.obs + src);
+        if constexpr (kXYZ3) T[t] = __ldg(a.z + src);
+    }
+    __syncthreads();
+    // Panel 0 into cur: thread t takes column t mod 16, every (kT/16)-th row.
+    gen_column<kXYZ3>(cur, 0, X, Y, Z, T, M, Mp, 0, min(kNB, M), tid & 15, tid >> 4, kT >> 4, *mp);
+    __syncthreads();
+
+    unsigned st = 0;  // thread 0: pivot flags
+    for (int p = 0; p < P; ++p) {
+        const int k0 = p * kNB, kb = min(kNB, M - k0);
+        const int n0 = k0 + kb;                    // first row / column of panel p+1
+        const int kb1 = max(0, min(kNB, M - n0));  // its width
+        if (warp == 0) {
+            st |= factor_phase(cur, M, k0, kb, mc, sh);
+        } else if (kb1 > 0) {
+            if constexpr (GEN != kGenClosed) {
+                const int u = tid - 32;
+                gen_column<kXYZ3>(nxt, n0, X, Y, Z, T, M, Mp, n0, kb1, u & 15, n0 + (u >> 4), (kT - 32) >> 4,
+                                  *mp);
+                update_warps_sync<NT>();
+                next_panel<false>(nxt, X, Y, Z, slab, M, p, n0, 1, kW - 1, mp);
+            } else {
+                next_panel<true>(nxt, X, Y, Z, slab, M, p, n0, 1, kW - 1, mp);
+            }
+        }
+        // The substitution needs only the factored diagonal block: warp 0
+        // publishes it (named barrier 3 over the CTA: warp 0 arrives, the
+        // others wait after their work on panel p+1) and goes on to its rows,
+        // which overlap the other warps' generation and update.
+        if (warp == 0) {
+            __syncwarp();
+            asm volatile("bar.arrive 3, %0;" ::"n"(NT) : "memory");
+        } else {
+            asm volatile("bar.sync 3, %0;" ::"n"(NT) : "memory");
+        }
+        // Rows below the diagonal block (after the 16 the factor warp solved
+        // for a full panel).  Warp 0, idle for most of the phase before,
+        // takes the first kSubstRows0 rows, the other warps the rest.
+        const int rs0 = k0 + (kb == kNB ? 2 * kNB : kb);
+        const int rw0 = min(Mp, rs0 + kSubstRows0);
+        const int rend = (warp == 0) ? rw0 : Mp;
+        for (int r = (warp == 0) ? rs0 + lane : rw0 + tid - 32; r < rend; r += (warp == 0) ? 32 : kT - 32)
+            solve_row(sh, cur + (r - k0) * 16, r);
+        __syncthreads();
+        // Panel p to the slab; panel p+1 takes panel p's update.
+        {
+            double *pg = slab + big_panel_base(p, Mp);
+            const double2 *s2 = reinterpret_cast<const double2 *>(cur);
+            double2 *g2 = reinterpret_cast<double2 *>(pg);
+            for (int e = tid; e < (Mp - k0) * 8; e += kT) g2[e] = s2[e];
+        }
+        if (kb1 > 0) last_update<NT>(nxt, cur, M, k0, n0);
+        __syncthreads();
+        double *t = cur;
+        cur = nxt;
+        nxt = t;
+    }
+
+    // log det of the conditional factor (positive pivots) and |u|^2 (row M).
+    double ld = 0.0, qf = 0.0;
+    for (int j = mc + tid; j < M; j += kT) {
+        const int q = j / kNB, c = j - q * kNB;
+        const double *pq = slab + big_panel_base(q, Mp);
+        const double dj = pq[(j - q * kNB) * 16 + swz(j, c)];
+        if (dj > 0) ld += log(dj * dj);
+        const double u = pq[(M - q * kNB) * 16 + swz(M, c)];
+        qf = fma(u, u, qf);
+    }
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+        ld += __shfl_xor_sync(0xffffffffu, ld, s);
+        qf += __shfl_xor_sync(0xffffffffu, qf, s);
+    }
+    if (lane == 0) {
+        sh.red[0][warp] = ld;
+        sh.red[1][warp] = qf;
+    }
+    if (warp == 0 && lane == 0 && st) atomicOr(&sh.status, st);
+    __syncthreads();
+    if (tid == 0) {
+        double Ls = 0.0, Qs = 0.0;
+        for (int w = 0; w < kW; ++w) {
+            Ls += sh.red[0][w];
+            Qs += sh.red[1][w];
+        }
+        const double v = -(Qs + Ls + (double)bs * a.log2pi) * 0.5;
+        unsigned s2 = sh.status;
+        if (!isfinite(v)) s2 |= BV_ST_NONFINITE;
+        a.block_llk[b] = v;
+        a.block_status[b] = s2 | a.status_or;
+    }
+}
+
+}  // namespace bv

@@ -17,7 +17,7 @@
 // the next batch's CTAs), and a completion thread per slot hands the results
 // back.
 //
-// Determinism.  Per-block work (process_block_big / run_block) and the
+// Determinism.  Per-block work (process_block_lean / run_block) and the
 // per-request reduction (reduce_blocks) are the code of the single-job path,
 // so a result is bit-identical to bv_llh_eval on the same layout under the
 // default schedule, alone or in any mix.
@@ -38,7 +38,7 @@
 
 #include "../../include/bv.h"
 #include "bv_common.cuh"
-#include "bv_llh_big.cuh"
+#include "bv_llh_lean.cuh"
 #include "bv_reduce.cuh"
 
 namespace bv {
@@ -92,10 +92,10 @@ __global__ void __launch_bounds__(kThreads, 1) llh_fp64_server_kernel(const JobD
 // The multi-CTA streamed kernel's server form: the same task list protocol
 // over the blocks whose two panels fit in shared memory (the rest run the
 // kernel above), NT threads per CTA, MINB CTAs per SM, one global slab per
-// CTA.  Per block the code of the handles' default path (process_block_big,
+// CTA.  Per block the code of the handles' default path (process_block_lean,
 // panel-by-panel generation), so a request's blocks give the bits a handle
 // created with the default schedule gives.
-template <int NT, int MINB>
+template <int NT, int MINB, int GEN>
 __global__ void __launch_bounds__(NT, MINB) llh_lean_server_kernel(const JobDesc *descs, const int2 *tasks,
                                                                    int ntasks, unsigned *counter,
                                                                    double *slab0, size_t slab_stride)
@@ -125,10 +125,7 @@ __global__ void __launch_bounds__(NT, MINB) llh_lean_server_kernel(const JobDesc
                 a.block_status[b] = a.status_or;
             }
         } else {
-            const MaternParams mp = d.mp;
-            process_block_big<NT, 64, LeanShared, 0, false, false>(a, mp, b,
-                                                                   reinterpret_cast<unsigned char *>(smem),
-                                                                   slab, sh);
+            process_block_lean<NT, GEN>(a, &d.mp, b, reinterpret_cast<unsigned char *>(smem), slab, sh);
         }
         __syncthreads();
         if (tid == 0) {
@@ -145,13 +142,15 @@ __global__ void __launch_bounds__(NT, MINB) llh_lean_server_kernel(const JobDesc
 }
 
 struct LeanServerVariant {
-    void (*kernel)(const JobDesc *, const int2 *, int, unsigned *, double *, size_t);
+    void (*kernel[2])(const JobDesc *, const int2 *, int, unsigned *, double *, size_t);  // by LeanGen
     int threads;
 };
+#define BV_LEAN_SERVER(NT, MINB) \
+    {{llh_lean_server_kernel<NT, MINB, kGenClosed>, llh_lean_server_kernel<NT, MINB, kGenGeneral>}, NT}
 static const LeanServerVariant kLeanServer[] = {
-    {llh_lean_server_kernel<128, 4>, 128},
-    {llh_lean_server_kernel<160, 3>, 160},
-    {llh_lean_server_kernel<256, 2>, 256},
+    BV_LEAN_SERVER(96, 4),
+    BV_LEAN_SERVER(128, 3),
+    BV_LEAN_SERVER(256, 2),
 };
 
 }  // namespace bv
@@ -228,7 +227,8 @@ bool grow_pinned(T *&p, size_t &cap, size_t need)
 struct bv_server {
     struct Slot {
         int index = 0;
-        cudaStream_t s = nullptr;
+        cudaStream_t s = nullptr, s2 = nullptr;       // s2: the general-nu launch beside the closed forms'
+        cudaEvent_t fork = nullptr, join = nullptr;
         // device
         double *bllk = nullptr;
         unsigned *bst = nullptr;
@@ -237,7 +237,7 @@ struct bv_server {
         size_t cap_tasks = 0;
         JobDesc *desc = nullptr;
         EvalResult *res = nullptr;
-        unsigned *counters = nullptr;  // [0]: work counter, [1 + r]: request r's done count
+        unsigned *counters = nullptr;  // [0]: work counter, [1 + r]: request r's done count, then two work counters
         double *slab = nullptr;
         size_t slab_stride = 0;
         int slab_max_m = 0;
@@ -389,13 +389,13 @@ struct LeanLaunch {
     int grid = 0;
 };
 
-bool lean_launch_for(const bv_server *S, int max_m, LeanLaunch &ll)
+bool lean_launch_for(const bv_server *S, int gen, int max_m, size_t blocks, LeanLaunch &ll)
 {
-    const int t = lean_table_threads(max_m);
-    ll.v = &kLeanServer[t == 128 ? 0 : (t == 160 ? 1 : 2)];
-    ll.smem = std::max<size_t>(big_layout(max_m, 64, 0, 0).total, kReduceScratchBytes);
+    const int t = lean_table_threads(gen, max_m, blocks);
+    ll.v = &kLeanServer[t == 96 ? 0 : (t == 128 ? 1 : 2)];
+    ll.smem = std::max<size_t>(big_layout(max_m, 0, 0, 0).total, kReduceScratchBytes);
     int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ll.v->kernel, ll.v->threads, ll.smem) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ll.v->kernel[gen], ll.v->threads, ll.smem) != cudaSuccess ||
         occ < 1) {
         cudaGetLastError();
         return false;
@@ -428,34 +428,47 @@ bool launch_batch(bv_server *S, bv_server::Slot &sl, const std::vector<Job *> &j
     // Tasks: merge the jobs' runs of equal M, largest M first.  Blocks above
     // the streamed kernel's limit (the first n_pers tasks) run the persistent
     // kernel, the others the streamed kernel, as under the handles' default
-    // schedule.
-    size_t n_pers = 0;
-    int pers_max_m = 0, lean_max_m = 0;
+    // schedule: the requests with a closed-form nu in one launch, those with
+    // a general nu in another beside it.
+    size_t n_pers = 0, n_lean[2] = {0, 0};
+    int pers_max_m = 0, lean_max_m[2] = {0, 0};
+    std::vector<int> gen(R);
+    for (int r = 0; r < R; ++r) {
+        fill_params(sl.h_desc[r].mp, rq[r].theta, jobs[r]->dist_scale);
+        gen[r] = sl.h_desc[r].mp.nu_kind == kNuGeneral ? kGenGeneral : kGenClosed;
+    }
     {
         std::vector<size_t> run(R, 0);
         size_t w = 0;
-        for (;;) {
+        // Pass 0: the persistent kernel's blocks; 1: closed forms; 2: general nu.
+        for (int pass = 0; pass < 3;) {
             int best = -1;
             for (int r = 0; r < R; ++r)
                 if (run[r] < jobs[r]->m_value.size() &&
+                    (pass == 0 ? jobs[r]->m_value[run[r]] > S->lean_limit : gen[r] == pass - 1) &&
                     (best < 0 || jobs[r]->m_value[run[r]] > jobs[best]->m_value[run[best]]))
                     best = r;
-            if (best < 0) break;
+            if (best < 0) {
+                ++pass;
+                continue;
+            }
+            const size_t w0 = w;
             const int m = jobs[best]->m_value[run[best]];
             for (int r = best; r < R; ++r) {
                 const Job &j = *jobs[r];
-                if (run[r] < j.m_value.size() && j.m_value[run[r]] == m) {
+                if (run[r] < j.m_value.size() && j.m_value[run[r]] == m && (pass == 0 || gen[r] == pass - 1)) {
                     const int b0 = j.m_start[run[r]];
                     const int b1 = (run[r] + 1 < j.m_start.size()) ? j.m_start[run[r] + 1] : j.bc;
                     for (int p = b0; p < b1; ++p) sl.h_tasks[w++] = make_int2(r, j.sorted[p]);
                     run[r]++;
                 }
             }
-            if (m > S->lean_limit) {
+            if (pass == 0) {
                 n_pers = w;
                 pers_max_m = std::max(pers_max_m, m);
             } else {
-                lean_max_m = std::max(lean_max_m, m);
+                n_lean[pass - 1] += w - w0;
+                lean_max_m[pass - 1] = std::max(lean_max_m[pass - 1], m);
             }
         }
         total = w;
@@ -476,19 +489,22 @@ bool launch_batch(bv_server *S, bv_server::Slot &sl, const std::vector<Job *> &j
             sl.slab = nullptr;
         }
     }
-    LeanLaunch ll;
-    if (ok && total > n_pers) {
-        ok = lean_launch_for(S, lean_max_m, ll);
-        ll.grid = std::max(1, std::min<int>(ll.grid, (int)(total - n_pers)));
-        const size_t bytes = ll.stride * 8 * (size_t)ll.grid;
-        if (ok && bytes > sl.lean_bytes) {
-            if (sl.lean_slab) cudaFreeAsync(sl.lean_slab, s);
-            ok = cudaMallocAsync(reinterpret_cast<void **>(&sl.lean_slab), bytes, s) == cudaSuccess;
-            sl.lean_bytes = ok ? bytes : 0;
-            if (!ok) {
-                cudaGetLastError();
-                sl.lean_slab = nullptr;
-            }
+    LeanLaunch ll[2];
+    size_t lean_bytes[2] = {0, 0};
+    for (int g = 0; ok && g < 2; ++g) {
+        if (n_lean[g] == 0) continue;
+        ok = lean_launch_for(S, g, lean_max_m[g], n_lean[g], ll[g]);
+        ll[g].grid = std::max(1, std::min<int>(ll[g].grid, (int)n_lean[g]));
+        lean_bytes[g] = ll[g].stride * 8 * (size_t)ll[g].grid;
+    }
+    if (ok && lean_bytes[0] + lean_bytes[1] > sl.lean_bytes) {
+        if (sl.lean_slab) cudaFreeAsync(sl.lean_slab, s);
+        sl.lean_bytes = lean_bytes[0] + lean_bytes[1];
+        ok = cudaMallocAsync(reinterpret_cast<void **>(&sl.lean_slab), sl.lean_bytes, s) == cudaSuccess;
+        if (!ok) {
+            cudaGetLastError();
+            sl.lean_slab = nullptr;
+            sl.lean_bytes = 0;
         }
     }
     if (!ok) {
@@ -521,12 +537,11 @@ bool launch_batch(bv_server *S, bv_server::Slot &sl, const std::vector<Job *> &j
         a.log2pi = std::log(2 * 3.141592653589793);
         a.mp = nullptr;
         a.task_begin = a.task_end = 0;
-        fill_params(d.mp, rq[r].theta, j.dist_scale);
         d.done = sl.counters + 1 + r;
         d.out = sl.res + r;
         off += j.bc;
     }
-    ok = cudaMemsetAsync(sl.counters, 0, (2 + R) * sizeof(unsigned), s) == cudaSuccess &&
+    ok = cudaMemsetAsync(sl.counters, 0, (3 + R) * sizeof(unsigned), s) == cudaSuccess &&
          cudaMemcpyAsync(sl.desc, sl.h_desc, R * sizeof(JobDesc), cudaMemcpyHostToDevice, s) == cudaSuccess &&
          cudaMemcpyAsync(sl.tasks, sl.h_tasks, total * sizeof(int2), cudaMemcpyHostToDevice, s) == cudaSuccess;
     if (ok && n_pers > 0) {
@@ -536,10 +551,24 @@ bool launch_batch(bv_server *S, bv_server::Slot &sl, const std::vector<Job *> &j
         kern<<<grid, kThreads, S->smem_bytes, s>>>(sl.desc, sl.tasks, (int)n_pers, sl.counters);
         ok = cudaGetLastError() == cudaSuccess;
     }
-    if (ok && ll.v) {
-        ll.v->kernel<<<ll.grid, ll.v->threads, ll.smem, s>>>(sl.desc, sl.tasks + n_pers, (int)(total - n_pers),
-                                                             sl.counters + 1 + R, sl.lean_slab, ll.stride);
+    // The general-nu launch on the slot's second stream: its CTAs take the
+    // SMs the closed forms' release (and both run at once where they fit).
+    const bool fork = ok && ll[0].v && ll[1].v;
+    if (fork)
+        ok = cudaEventRecord(sl.fork, s) == cudaSuccess && cudaStreamWaitEvent(sl.s2, sl.fork, 0) == cudaSuccess;
+    for (int g = 0; ok && g < 2; ++g) {
+        if (!ll[g].v) continue;
+        cudaStream_t gs = (fork && g == 1) ? sl.s2 : s;
+        ll[g].v->kernel[g]<<<ll[g].grid, ll[g].v->threads, ll[g].smem, gs>>>(
+            sl.desc, sl.tasks + n_pers + (g ? n_lean[0] : 0), (int)n_lean[g], sl.counters + 1 + R + g,
+            sl.lean_slab + (g ? lean_bytes[0] / 8 : 0), ll[g].stride);
         ok = cudaGetLastError() == cudaSuccess;
+    }
+    if (fork) {
+        // Joined whatever happened, so that nothing of the batch outlives it.
+        const bool joined = cudaEventRecord(sl.join, sl.s2) == cudaSuccess &&
+                            cudaStreamWaitEvent(s, sl.join, 0) == cudaSuccess;
+        ok = ok && joined;
     }
     ok = ok && cudaMemcpyAsync(sl.h_res, sl.res, R * sizeof(EvalResult), cudaMemcpyDeviceToHost, s) ==
                    cudaSuccess;
@@ -684,6 +713,7 @@ void completer_main(bv_server *S, bv_server::Slot *sl)
 
 void destroy_slot(bv_server::Slot &sl)
 {
+    if (sl.s2) cudaStreamSynchronize(sl.s2);
     if (sl.s) cudaStreamSynchronize(sl.s);
     cudaFree(sl.bllk);
     cudaFree(sl.bst);
@@ -697,6 +727,9 @@ void destroy_slot(bv_server::Slot &sl)
     cudaFreeHost(sl.h_desc);
     cudaFreeHost(sl.h_res);
     if (sl.s) cudaStreamDestroy(sl.s);
+    if (sl.s2) cudaStreamDestroy(sl.s2);
+    if (sl.fork) cudaEventDestroy(sl.fork);
+    if (sl.join) cudaEventDestroy(sl.join);
 }
 
 }  // namespace
@@ -769,11 +802,12 @@ extern "C" int bv_server_create(const bv_server_opts *opts, bv_server **out)
     // The streamed kernel: the handles' limit, and its shared memory allowed.
     {
         cudaFuncAttributes fl;
-        BV_CUDA_TRY(cudaFuncGetAttributes(&fl, kLeanServer[2].kernel));
+        BV_CUDA_TRY(cudaFuncGetAttributes(&fl, kLeanServer[2].kernel[kGenClosed]));
         const size_t avail = (size_t)optin - fl.sharedSizeBytes;
-        S->lean_limit = big_max_m_for_bytes(avail, 64, 0, 0);
+        S->lean_limit = big_max_m_for_bytes(avail, 0, 0, 0);
         for (const LeanServerVariant &v : kLeanServer)
-            BV_CUDA_TRY(cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)avail));
+            for (auto k : v.kernel)
+                BV_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)avail));
     }
     BV_CUDA_TRY(cudaStreamCreateWithFlags(&S->upload, cudaStreamNonBlocking));
     for (int k = 0; k < S->opts.max_inflight; ++k) {
@@ -781,18 +815,25 @@ extern "C" int bv_server_create(const bv_server_opts *opts, bv_server **out)
         sl->index = k;
         const int R = S->opts.max_batch;
         BV_CUDA_TRY(cudaStreamCreateWithFlags(&sl->s, cudaStreamNonBlocking));
+        BV_CUDA_TRY(cudaStreamCreateWithFlags(&sl->s2, cudaStreamNonBlocking));
+        BV_CUDA_TRY(cudaEventCreateWithFlags(&sl->fork, cudaEventDisableTiming));
+        BV_CUDA_TRY(cudaEventCreateWithFlags(&sl->join, cudaEventDisableTiming));
         BV_CUDA_TRY(cudaMalloc(&sl->desc, R * sizeof(JobDesc)));
         BV_CUDA_TRY(cudaMalloc(&sl->res, R * sizeof(EvalResult)));
-        BV_CUDA_TRY(cudaMalloc(&sl->counters, (2 + R) * sizeof(unsigned)));
+        BV_CUDA_TRY(cudaMalloc(&sl->counters, (3 + R) * sizeof(unsigned)));
         BV_CUDA_TRY(cudaHostAlloc(&sl->h_desc, R * sizeof(JobDesc), cudaHostAllocDefault));
         BV_CUDA_TRY(cudaHostAlloc(&sl->h_res, R * sizeof(EvalResult), cudaHostAllocDefault));
         // Streamed-kernel slabs for blocks up to M = 350 (cs = 300 with
         // blocks of 50) at every table point, so that batches of such jobs
         // allocate nothing; larger batches grow them.
         size_t pre = 0;
-        for (int m : {170, 250, std::min(350, S->lean_limit)}) {
-            LeanLaunch ll;
-            if (lean_launch_for(S.get(), m, ll)) pre = std::max(pre, ll.stride * 8 * (size_t)ll.grid);
+        for (int m : {115, 250, std::min(350, S->lean_limit)}) {
+            size_t both = 0;
+            for (int g = 0; g < 2; ++g) {
+                LeanLaunch ll;
+                if (lean_launch_for(S.get(), g, m, 1 << 20, ll)) both += ll.stride * 8 * (size_t)ll.grid;
+            }
+            pre = std::max(pre, both);
         }
         if (pre > 0) {
             BV_CUDA_TRY(cudaMalloc(&sl->lean_slab, pre));

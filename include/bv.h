@@ -171,11 +171,9 @@ typedef struct {
     int streamed_threads; /* threads per CTA of that kernel (0: none)       */
     int streamed_variant; /* its variant, an index into tune_ms             */
     double tune_ms[6];   /* with bv_opts.tune: the streamed kernel's time on
-                            the first evaluation per variant: 96 x 5 CTAs per
-                            SM, 160 x 3, 256 x 2 and 128 x 4 threads per CTA
-                            generating panel by panel, then 160 x 3 and
-                            256 x 2 generating the whole matrix first (0
-                            where not timed)                                 */
+                            the first evaluation per variant: 96 threads x 4
+                            CTAs per SM, 160 x 3, 256 x 2, 128 x 3, 160 x 2
+                            and 256 x 1 (0 where not timed)                  */
 } bv_status;
 
 typedef struct bv_handle bv_handle;
