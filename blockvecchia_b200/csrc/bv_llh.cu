@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(NT, MINB) llh_lean_kernel_t(LlhArgs a)
                 a.block_status[b] = a.status_or;
             }
         } else {
-            process_block_lean<NT, GEN>(a, a.mp, b, reinterpret_cast<unsigned char *>(smem), slab, sh);
+            process_block_lean<NT, MINB, GEN>(a, a.mp, b, reinterpret_cast<unsigned char *>(smem), slab, sh);
         }
         __syncthreads();
     }
@@ -96,19 +96,25 @@ struct LeanVariant {
     void (*kernel[3])(LlhArgs);  // by LeanGen
     int threads;
 };
-#define BV_LEAN(NT, MINB)                                                                          \
+#define BV_LEAN(NT, MINB, MINB3)                                                                   \
     {{llh_lean_kernel_t<NT, MINB, kGenClosed>, llh_lean_kernel_t<NT, MINB, kGenGeneral>,          \
-      llh_lean_kernel_t<NT, MINB, kGenXYZ>}, NT}
-// The table's three sizes and three others (lean_table_threads has the
-// measurements).  All give the same bits, so bv_opts.tune may pick any.
+      llh_lean_kernel_t<NT, MINB3, kGenXYZ>}, NT}
+// The table's four and two others (lean_table_threads has the measurements).  All give the same bits, so bv_opts.tune may pick any.
 static const LeanVariant kLeanVariants[] = {
-    BV_LEAN(96, 4), BV_LEAN(160, 3), BV_LEAN(256, 2), BV_LEAN(128, 3), BV_LEAN(160, 2), BV_LEAN(256, 1),
+    BV_LEAN(96, 4, 5),  BV_LEAN(160, 3, 3), BV_LEAN(256, 2, 2),
+    BV_LEAN(128, 3, 4), BV_LEAN(160, 2, 2), BV_LEAN(256, 1, 1),
 };
 constexpr int kNumLean = (int)(sizeof(kLeanVariants) / sizeof(kLeanVariants[0]));
 static int lean_variant(int gen, int max_m, size_t blocks)
 {
     const int t = lean_table_threads(gen, max_m, blocks);
-    return t == 96 ? 0 : (t == 128 ? 3 : 2);
+    return t == 96 ? 0 : (t == 128 ? 3 : (t == 160 ? 4 : 2));
+}
+
+__global__ void __launch_bounds__(kTabThreads) ktab_kernel(const MaternParams *mp, double2 *tab)
+{
+    const int idx = (int)(blockIdx.x * kTabThreads + threadIdx.x) >> 4;
+    if (idx < kTabN && mp->kt_on) ktab_build_interval(*mp, idx, tab);
 }
 
 static thread_local char g_err[1024] = "";
@@ -162,6 +168,7 @@ struct bv_handle {
     bool tuned = false;
     double tune_ms[kNumLean] = {};
     MaternParams *d_mp = nullptr;
+    double2 *d_ktab = nullptr;  // the general-nu table (bv_ktab.cuh)
     EvalResult *d_res = nullptr;
     MixedWork mixed;  // mixed-precision scratch (bv_llh_mixed.cuh)
     // pinned host
@@ -227,6 +234,7 @@ static void handle_free(bv_handle *h)
     cudaFree(h->d_slab);
     cudaFree(h->d_slab_lean);
     cudaFree(h->d_mp);
+    cudaFree(h->d_ktab);
     cudaFree(h->d_res);
     mixed_free(h->mixed);
     cudaFreeHost(h->h_mp);
@@ -416,9 +424,9 @@ static int plan_lean_launch(bv_handle *h, const cudaDeviceProp &prop, int begin,
         const LeanVariant &v = kLeanVariants[k.variant];
         k.fn = v.kernel[gen];
         k.threads = v.threads;
-        k.smem = big_layout(max_m, 0, h->nz, 0).total;
         cudaFuncAttributes fa;
         BV_CUDA_TRY(cudaFuncGetAttributes(&fa, k.fn));
+        k.smem = lean_smem(gen, max_m, h->nz, (size_t)optin - fa.sharedSizeBytes);
         if (k.smem > (size_t)optin - fa.sharedSizeBytes) {
             set_error("plan: blocks of M = %d exceed the streamed schedule's shared memory", max_m);
             return BV_E_TOOLARGE;
@@ -593,6 +601,10 @@ static int enqueue_eval(bv_handle *h, cudaStream_t s, int kind)
     BV_CUDA_TRY(cudaMemcpyAsync(h->d_mp, h->h_mp, sizeof(MaternParams), cudaMemcpyHostToDevice, s));
     BV_CUDA_TRY(cudaMemsetAsync(h->d_counters, 0, sizeof(unsigned) * std::max<size_t>(1, h->launches.size()), s));
     BV_CUDA_TRY(record_timing(h->evk0, s));
+    if (kind == 1) {
+        ktab_kernel<<<kTabCtas, kTabThreads, 0, s>>>(h->d_mp, h->d_ktab);
+        BV_CUDA_TRY(cudaGetLastError());
+    }
     auto fp64_args = [&](unsigned *counter, const int *order, int begin, int end) {
         LlhArgs a{};
         a.x = h->d_x;
@@ -614,6 +626,7 @@ static int enqueue_eval(bv_handle *h, cudaStream_t s, int kind)
         a.big_max_m = h->use_big ? h->big_max_m : 0;
         a.log2pi = std::log(2 * 3.141592653589793);
         a.mp = h->d_mp;
+        a.ktab = h->d_ktab;
         a.task_begin = begin;
         a.task_end = end;
         return a;
@@ -792,6 +805,7 @@ extern "C" int bv_create(const bv_layout *L, const bv_opts *opts, bv_handle **ou
     BV_CUDA_H(cudaMalloc(&h->d_block_llk, bc * sizeof(double)));
     BV_CUDA_H(cudaMalloc(&h->d_block_status, bc * sizeof(unsigned)));
     BV_CUDA_H(cudaMalloc(&h->d_mp, sizeof(MaternParams)));
+    BV_CUDA_H(cudaMalloc(&h->d_ktab, kTabEntries * sizeof(double2)));
     BV_CUDA_H(cudaMalloc(&h->d_res, sizeof(EvalResult)));
     BV_CUDA_H(cudaMallocHost(&h->h_mp, sizeof(MaternParams)));
     BV_CUDA_H(cudaMallocHost(&h->h_res, sizeof(EvalResult)));
@@ -901,6 +915,7 @@ static int fill_params(bv_handle *h, const double *theta)
     p.nu_kind = (nu == 0.5) ? kNuHalf : (nu == 1.5) ? kNuThreeHalves : (nu == 2.5) ? kNuFiveHalves
                                                                                   : kNuGeneral;
     matern_prepare(p);
+    ktab_prepare(p);
     return BV_OK;
 }
 

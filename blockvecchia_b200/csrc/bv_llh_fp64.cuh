@@ -33,6 +33,7 @@
 
 #include <stdint.h>
 
+#include "bv_ktab.cuh"
 #include "bv_matern.cuh"
 
 namespace bv {
@@ -62,6 +63,7 @@ struct LlhArgs {
     int task_begin, task_end;   // slice of `order` this launch serves
     const int *task_count;      // if set, the slice also ends at *task_count (device)
     unsigned status_or;         // flags OR-ed into every block status written
+    const double2 *ktab;        // this evaluation's general-nu table (streamed kernel), or nullptr
     int big_max_m;              // blocks with smem_max_m < M <= big_max_m: streamed path
 };
 

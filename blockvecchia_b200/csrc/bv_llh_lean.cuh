@@ -29,26 +29,35 @@
 
 namespace bv {
 
-// How a block's entries are generated: the closed forms on 2-D locations in
-// the update warps' accumulators; a general nu (K_nu) and locations with a
-// third coordinate (cov_xyz), which are long, through shared memory.  Each is
-// a kernel of its own: with the long ones beside it (inlined or called) the
-// closed forms' kernel spills 500-900 bytes per thread (n = 1M, cs = 200: 55
-// against 44 ms).
+// How a block's entries are generated: on 2-D locations in the update warps'
+// accumulators, the closed forms and (through the table) a general nu; with a
+// third coordinate (cov_xyz, long) through shared memory.  Each is a kernel of
+// its own: with a call of K_nu beside it (inlined or not) the closed forms'
+// kernel spills 500-900 bytes per thread (n = 1M, cs = 200: 55 against 44 ms).
 enum LeanGen : int { kGenClosed = 0, kGenGeneral = 1, kGenXYZ = 2 };
 
+// Dynamic shared memory of a launch whose largest block has M = max_m; a
+// general nu takes the table's window too where it fits in `avail` (a block
+// without room for it reads the table from global memory).
+inline size_t lean_smem(int gen, int max_m, int nz, size_t avail)
+{
+    const size_t b = big_layout(max_m, 0, nz, 0).total;
+    return gen == kGenGeneral ? std::max(b, std::min(avail, b + kTabWinBytes)) : b;
+}
+
 // CTA size of the streamed kernel for a launch of `blocks` blocks, the largest
-// of M = max_m (the handles and the server use it).  Multiples of 128 threads
-// keep warp 0, whose pivot chain is the block's critical path, on an SM
-// sub-partition without update warps: a warp issuing FP64 MMAs back to back
-// beside the chain stretched it from 5.2k to 16.9k cycles per panel.  Below M ~
-// 115 the panels leave an update warp too few tiles, and 96 threads with four
-// CTAs per SM win; beyond M ~ 240 only two CTAs' panels fit an SM, and 256
-// threads give them as many update warps as registers allow.  A launch that
-// leaves SMs with one or two blocks wants each block short: 128 threads.
-// Entries generated through shared memory are a larger share of the update
-// warps' work: more of them.  Kernel ms at 96 x 4 CTAs per SM / 160 x 3 /
-// 256 x 2 / 128 x 3 / 160 x 2:
+// of M = max_m (the handles and the server use it).  128 threads keep warp 0,
+// whose pivot chain is the block's critical path, on an SM sub-partition
+// without update warps: a warp issuing FP64 MMAs back to back beside the
+// chain stretched it from 5.2k to 16.9k cycles per panel.  Below M ~ 115 the
+// panels leave an update warp too few tiles, and 96 threads with four CTAs
+// per SM win; a launch of at most one wave of 128-thread CTAs wants each
+// block short instead, and one that 96-thread CTAs finish in one wave takes
+// those.  Beyond M ~ 240 only two CTAs' panels fit an SM: 160 threads without
+// spills, or 256 where few waves of blocks make the last one count.  Entries
+// generated through shared memory (a third coordinate) are a larger share of
+// the update warps' work: more of them.  Kernel ms at 96 x 4 CTAs per SM /
+// 160 x 3 / 256 x 2 / 128 x 3 / 160 x 2:
 //   cs =  30, classic, 30k blocks (M <=  31): 0.55 / 0.94 / 1.30 / 0.66 / 0.96
 //   cs =  60, 150 blocks (M <=  82):          .042 / .047 / .045 / .036 / .037
 //   cs =  60, 5k blocks (M <=  77):           0.27 / 0.42 / 0.55 / 0.30 / 0.39
@@ -57,13 +66,26 @@ enum LeanGen : int { kGenClosed = 0, kGenGeneral = 1, kGenXYZ = 2 };
 //   cs = 160, 10k blocks (M <= 177):          2.74 / 3.20 / 3.40 / 2.66 / 2.85
 //   cs = 200, 100k blocks (M <= 217):         53.1 / 50.9 / 48.8 / 44.0 / 45.5
 //   cs = 240, 10k blocks (M <= 257):          7.29 / 6.96 / 6.68 / 6.19 / 6.09
-//   cs = 300, 1.5k blocks (M <= 322):         2.69 / 1.93 / 1.73 / 1.96 / 1.76
-//   space-time, cs = 100, 2.5k (M <= 114):    1.26 / 1.00 / 0.99 / 1.13 / 1.28
-//   nu = 0.8, cs = 120, 10k (M <= 137):       7.86 / 6.46 / 5.92 / 7.19 / 7.56
+//   cs = 300, 1.5k blocks (M <= 322):         2.68 / 1.89 / 1.64 / 1.96 / 1.76
+//   cs = 300, 20k blocks (M <= 317):          30.9 / 21.7 / 20.8 / 22.8 / 19.7
+//   nu = 0.8, cs =  80, 10k (M <=  97):       1.07 / 1.44 / 1.74 / 1.11 / 1.35
+//   nu = 0.8, cs = 120, 10k (M <= 137):       2.11 / 2.64 / 2.87 / 2.03 / 2.36
+//   nu = 0.8, cs = 200, 10k (M <= 217):       5.55 / 7.00 / 6.32 / 4.86 / 5.38
+//   nu = 0.8, cs = 300, 20k (M <= 317):       34.1 / 32.7 / 27.2 / 26.1 / 25.1
+// and for a third coordinate at 96 x 5 / 160 x 3 / 256 x 2 / 128 x 4 / 160 x 2:
+//   cs =  30, 2.5k blocks (M <=  44):         0.21 / 0.22 / 0.27 / 0.21 / 0.27
+//   cs =  47, 250 blocks (M <=  61):          .103 / .065 / .058 / .077 / .062
+//   cs =  60, 500 blocks (M <=  74):          .144 / .144 / .129 / .124 / .142
+//   cs =  60, 2.5k blocks (M <=  74):         0.53 / 0.48 / 0.51 / 0.49 / 0.60
+//   cs = 100, 2.5k blocks (M <= 114):         1.13 / 0.98 / 0.98 / 1.02 / 1.28
+//   cs = 200, 2.5k blocks (M <= 214):         5.40 / 3.24 / 3.07 / 3.98 / 4.30
 inline int lean_table_threads(int gen, int max_m, size_t blocks)
 {
-    if (max_m > 250 || gen != kGenClosed) return 256;
-    return (max_m <= 115 && blocks > 600) ? 96 : 128;
+    constexpr size_t sms = 148;
+    if (gen == kGenXYZ) return (max_m <= 90 && blocks > 2 * sms) ? 128 : 256;
+    if (max_m > 250) return (gen == kGenClosed && blocks < 16 * sms) ? 256 : 160;
+    if (max_m <= 115) return blocks > 3 * sms ? 96 : 128;
+    return (max_m <= 180 && blocks > 3 * sms && blocks <= 4 * sms) ? 160 : 128;
 }
 
 // The static shared scratch the streamed path needs (a subset of
@@ -187,6 +209,84 @@ __device__ __forceinline__ void gen_tiles(double (&d)[NTILE][2][2], const double
     }
 }
 
+// The general-nu table's part in shared memory for one block: octaves
+// [base / 8, base / 8 + kTabWinOct) of the squared distance's exponent field.
+struct KWindow {
+    const double2 *win;  // [kTabPairs][kTabWinN]; nullptr: no room for it
+    const double2 *tab;  // the whole table, in global memory
+    int base;            // (exponent field << 3) of the window's first interval
+};
+
+// The same entries for a general nu, through the table (bv_ktab.cuh): the
+// squared distance's exponent and top three mantissa bits give the interval.
+// The loads are 16-byte shared-memory reads at random intervals (about three
+// wavefronts per quarter-warp), the lanes' polynomials independent chains.
+template <int NTILE>
+__device__ __forceinline__ void gen_tiles_table(double (&d)[NTILE][2][2], const double *X, const double *Y,
+                                                const double *Z, int M, int n0, int i0, int rstep,
+                                                const TileLane &L, const MaternParams *mp, const KWindow &kw)
+{
+    double s[NTILE][4], t[NTILE][4];
+    int k[NTILE][4];
+    unsigned out = 0;  // entries of this lane outside the window
+    {
+        double xj[4], yj[4];
+#pragma unroll
+        for (int nj = 0; nj < 2; ++nj) {
+            const double2 a = ld2(X + n0 + 8 * nj + 2 * L.c4), b = ld2(Y + n0 + 8 * nj + 2 * L.c4);
+            xj[2 * nj] = a.x;
+            xj[2 * nj + 1] = a.y;
+            yj[2 * nj] = b.x;
+            yj[2 * nj + 1] = b.y;
+        }
+#pragma unroll
+        for (int m = 0; m < NTILE; ++m) {
+            const int i = min(i0 + m * rstep + L.r8, M - 1);
+            const double xi = X[i], yi = Y[i];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const double dx = xj[c] - xi, dy = yj[c] - yi;
+                s[m][c] = __fma_rn(dx, dx, __dmul_rn(dy, dy));
+                const int kk = (__double2hiint(s[m][c]) >> 17) - kw.base;
+                const bool in = (unsigned)kk < (unsigned)kTabWinN;
+                if (!in && s[m][c] != 0.0) out |= 1u << (4 * m + c);
+                k[m][c] = in ? kk : 0;
+                t[m][c] = ktab_t(s[m][c], 3);
+                d[m][c >> 1][c & 1] = 0.0;
+            }
+        }
+    }
+    if (kw.win) {
+#pragma unroll
+        for (int h = kTabPairs - 1; h >= 0; --h)
+#pragma unroll
+            for (int m = 0; m < NTILE; ++m)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const double2 q = kw.win[h * kTabWinN + k[m][c]];
+                    double &v = d[m][c >> 1][c & 1];
+                    v = fma(fma(v, t[m][c], q.y), t[m][c], q.x);
+                }
+    } else {
+        out = (1u << (4 * NTILE)) - 1;
+    }
+    const double sigma2 = __ldg(&mp->sigma2), nugget = __ldg(&mp->nugget);
+    const bool any = __any_sync(0xffffffffu, out != 0);
+#pragma unroll
+    for (int m = 0; m < NTILE; ++m) {
+        const int i = i0 + m * rstep + L.r8;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int j = n0 + 8 * (c >> 1) + 2 * L.c4 + (c & 1);
+            double &v = d[m][c >> 1][c & 1];
+            if (any && (out >> (4 * m + c) & 1u)) v = ktab_entry(s[m][c], mp, kw.tab);
+            if (s[m][c] == 0.0) v = -sigma2;
+            if (i >= M) v = (i == M) ? -Z[j] : 0.0;
+            else if (j >= i) v = (j == i) ? __dsub_rn(v, nugget) : 0.0;
+        }
+    }
+}
+
 // Fragments of one slab panel for a group of NTILE tiles: B, the 16 rows n0..
 // that every tile of the panel multiplies by, through L1 (n = 1M, cs = 200:
 // 51.2 against 51.8 ms through L2 only); A, each tile's own rows, read once
@@ -232,7 +332,7 @@ template <int NTILE>
 __device__ __forceinline__ void update_tiles(double (&d)[NTILE][2][2], const double *slab, int Mp, int p,
                                              int n0, int i0, int rstep, const TileLane &L)
 {
-    if (p == 0) return;
+    if (p <= 0) return;
     const double *pb = slab + 16 * (n0 + L.r8), *pa = slab + 16 * (i0 + L.r8);
     const int tstep = 16 * rstep;
     int step = 16 * (Mp - 16);  // from panel q to q + 1
@@ -258,19 +358,21 @@ __device__ __forceinline__ void update_tiles(double (&d)[NTILE][2][2], const dou
     }
 }
 
-// Panel p+1 (rows n0..): its tiles evaluated by the lanes that hold them
-// (kGen) or read from the shared panel (generated there, positive), panels
-// 0..p-1 applied, the negated entries into nxt.  Warps [w0, w0 + nw) take
-// tiles t, t + nw, ...
-template <int NTILE, bool kGen>
+// Panel p+1 (rows n0..): its tiles evaluated by the lanes that hold them, or
+// (kGenXYZ) read from the shared panel (generated there, positive), panels
+// 0..p-1 applied, the negated entries into nxt; panel 0 (p = -1, a general
+// nu) in its own sign.  Warps [w0, w0 + nw) take tiles t, t + nw, ...
+template <int NTILE, int GEN>
 __device__ __forceinline__ void next_tiles(double *nxt, const double *X, const double *Y, const double *Z,
                                            const double *slab, int M, int p, int n0, int t0, int nw,
-                                           const TileLane &L, const MaternParams *mp)
+                                           const TileLane &L, const MaternParams *mp, const KWindow &kw)
 {
     const int Mp = M + 1, i0 = n0 + 8 * t0, rstep = 8 * nw;
     double d[NTILE][2][2];
-    if constexpr (kGen) {
+    if constexpr (GEN == kGenClosed) {
         gen_tiles<NTILE>(d, X, Y, Z, M, n0, i0, rstep, L, mp);
+    } else if constexpr (GEN == kGenGeneral) {
+        gen_tiles_table<NTILE>(d, X, Y, Z, M, n0, i0, rstep, L, mp, kw);
     } else {
 #pragma unroll
         for (int m = 0; m < NTILE; ++m) {
@@ -284,6 +386,15 @@ __device__ __forceinline__ void next_tiles(double *nxt, const double *X, const d
         }
     }
     update_tiles<NTILE>(d, slab, Mp, p, n0, i0, rstep, L);
+    if (GEN == kGenGeneral && p < 0) {
+#pragma unroll
+        for (int m = 0; m < NTILE; ++m)
+#pragma unroll
+            for (int nj = 0; nj < 2; ++nj) {
+                d[m][nj][0] = -d[m][nj][0];
+                d[m][nj][1] = -d[m][nj][1];
+            }
+    }
 #pragma unroll
     for (int m = 0; m < NTILE; ++m) {
         const int i = i0 + m * rstep + L.r8;
@@ -295,18 +406,18 @@ __device__ __forceinline__ void next_tiles(double *nxt, const double *X, const d
     }
 }
 
-template <bool kGen>
+template <int GEN>
 __device__ __forceinline__ void next_panel(double *nxt, const double *X, const double *Y, const double *Z,
                                            const double *slab, int M, int p, int n0, int w0, int nw,
-                                           const MaternParams *mp)
+                                           const MaternParams *mp, const KWindow &kw)
 {
     const TileLane L;
     const int ntiles = (M + 8 - n0) >> 3;  // rows n0..M
     for (int t0 = (threadIdx.x >> 5) - w0; t0 < ntiles; t0 += nw * kDT) {
         if (t0 + nw < ntiles)
-            next_tiles<kDT, kGen>(nxt, X, Y, Z, slab, M, p, n0, t0, nw, L, mp);
+            next_tiles<kDT, GEN>(nxt, X, Y, Z, slab, M, p, n0, t0, nw, L, mp, kw);
         else
-            next_tiles<1, kGen>(nxt, X, Y, Z, slab, M, p, n0, t0, nw, L, mp);
+            next_tiles<1, GEN>(nxt, X, Y, Z, slab, M, p, n0, t0, nw, L, mp, kw);
     }
 }
 
@@ -440,10 +551,9 @@ __device__ __forceinline__ unsigned factor_panel(int k0, int kb, int mc, double 
             e[3] = make_double2(g3[1], g3[2]);
         }
         __syncwarp();
-        const double2 e1 = ld2(&ex[1][0]);
-        const double2 e2a = ld2(&ex[2][0]), e2b = ld2(&ex[2][2]);
-        const double2 e3a = ld2(&ex[3][0]), e3b = ld2(&ex[3][2]), e3c = ld2(&ex[3][4]), e3d = ld2(&ex[3][6]);
-        const double e0 = ex[0][0], e2c = ex[2][4];
+        // Read in two parts: all at once would spill at 128 registers.
+        const double e0 = ex[0][0];
+        const double2 e1 = ld2(&ex[1][0]), e2a = ld2(&ex[2][0]), e3a = ld2(&ex[3][0]);
         double piv[4], inv[4], w[4];
         bool ok[4];
         // A failed pivot's column is zero below it; rsqrt of 1 keeps the
@@ -460,6 +570,9 @@ __device__ __forceinline__ unsigned factor_panel(int k0, int kb, int mc, double 
         pivot(1, fma(-l10, l10, e1.y));
         const double l21 = fma(-l20, l10, e2a.y) * inv[1], l31 = fma(-l30, l10, e3a.y) * inv[1];
         w[1] = fma(-w[0], l10, s1) * inv[1];
+        asm volatile("" ::: "memory");
+        const double2 e2b = ld2(&ex[2][2]), e3b = ld2(&ex[3][2]), e3c = ld2(&ex[3][4]), e3d = ld2(&ex[3][6]);
+        const double e2c = ex[2][4];
         pivot(2, fma(-l21, l21, (fma(-l20, l20, e2b.x) + e2b.y) + e2c));
         const double l32 = fma(-l31, l21, (fma(-l30, l20, e3b.x) + e3b.y) + e3c.x) * inv[2];
         w[2] = fma(-w[1], l21, (fma(-w[0], l20, g2[0]) + g2[1]) + g2[2]) * inv[2];
@@ -479,9 +592,51 @@ __device__ __forceinline__ unsigned factor_panel(int k0, int kb, int mc, double 
     return st;
 }
 
+// The same with one column at a time and shuffles, in half the registers (62
+// against 110: no spills in kernels limited to 128; 3.6k cycles per panel
+// alone, more than factor_panel's when the shared-memory pipe is loaded).
+__device__ __forceinline__ unsigned factor_panel_narrow(int k0, int kb, int mc, double (&v)[kNB],
+                                                        double &myinv, double (*Lt)[kNB])
+{
+    const int lane = threadIdx.x & 31;
+    const bool low = lane < kNB;
+    unsigned st = 0;
+    myinv = 0.0;
+    double pre = v[0];
+#pragma unroll
+    for (int q = 0; q < kNB; ++q) {
+        const double preq = __shfl_sync(0xffffffffu, pre, q);
+        double s = pre, piv = preq;
+        if (q > 0) {
+            const double l = __shfl_sync(0xffffffffu, v[q - 1], q);
+            s = fma(-v[q - 1], l, s);
+            piv = fma(-l, l, preq);
+        }
+        const bool ok = piv > 0.0;
+        double inv = rsqrt(ok ? piv : 1.0);
+        inv = ok ? inv : 0.0;
+        if (q + 1 < kNB) {
+            double s4[4] = {v[q + 1], 0.0, 0.0, 0.0};
+#pragma unroll
+            for (int k = 0; k < q; ++k) {
+                const double lk = __shfl_sync(0xffffffffu, v[k], q + 1);
+                s4[k & 3] = fma(-v[k], lk, s4[k & 3]);
+            }
+            pre = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+        }
+        if (!ok && q < kb) st |= (k0 + q < mc) ? 1u : 2u;
+        const double dq = ok ? piv * inv : piv;
+        v[q] = (lane > q) ? s * inv : ((lane == q) ? dq : v[q]);
+        if (lane == q) myinv = inv;
+        if (low) Lt[q][lane] = (lane < kb) ? v[q] : 0.0;
+    }
+    return st;
+}
+
 // The factor warp's part of panel p (rows k0.. in cur): lane r < kb owns row
 // k0+r of the diagonal block; with a full panel the upper lanes solve the
 // next 16 rows on the same chain, so the substitution starts 16 rows on.
+template <bool kNarrow>
 __device__ __forceinline__ unsigned factor_phase(double *cur, int M, int k0, int kb, int mc, LeanShared &sh)
 {
     const int lane = threadIdx.x & 31;
@@ -494,7 +649,11 @@ __device__ __forceinline__ unsigned factor_phase(double *cur, int M, int k0, int
 #pragma unroll
     for (int c = 0; c < kNB; ++c)
         if (!(valid && c < kb && (!low || c <= lane))) v[c] = 0.0;
-    const unsigned st = factor_panel(k0, kb, mc, v, myinv, sh.Lt, sh.ex);
+    unsigned st;
+    if constexpr (kNarrow)
+        st = factor_panel_narrow(k0, kb, mc, v, myinv, sh.Lt);
+    else
+        st = factor_panel(k0, kb, mc, v, myinv, sh.Lt, sh.ex);
     if (valid) store_row(rowp, row, v);
     if (low) sh.inv[lane] = (lane < kb) ? myinv : 0.0;
     return st;
@@ -533,7 +692,7 @@ __device__ __forceinline__ void solve_row(const LeanShared &sh, double *row, int
 // and solves, the other NT/32 - 1 warps generate and update).  smem: the
 // dynamic area (big_layout(M, 0, nz, 0).total bytes); slab: this CTA's global
 // slab (big_slab_doubles(M) doubles).
-template <int NT, int GEN>
+template <int NT, int MINB, int GEN>
 __device__ __forceinline__ void process_block_lean(const LlhArgs &a, const MaternParams *mp, int b,
                                                           unsigned char *smem, double *slab, LeanShared &sh)
 {
@@ -554,36 +713,90 @@ __device__ __forceinline__ void process_block_lean(const LlhArgs &a, const Mater
     double *cur = reinterpret_cast<double *>(smem + l.o_cur);
     double *nxt = reinterpret_cast<double *>(smem + l.o_next);
 
+    // For the table the pad to whole panels repeats the last point (its
+    // entries are never used, but stay in the range of the block's).
     const int *kidx = a.knn + (size_t)b * a.cs;
-    for (int t = tid; t < M; t += kT) {
-        const int src = (t < mc) ? __ldg(kidx + t) : off + (t - mc);
+    for (int t = tid; t < (GEN == kGenGeneral ? P * kNB : M); t += kT) {
+        const int u = (GEN == kGenGeneral) ? min(t, M - 1) : t;
+        const int src = (u < mc) ? __ldg(kidx + u) : off + (u - mc);
         X[t] = __ldg(a.x + src);
         Y[t] = __ldg(a.y + src);
         Z[t] = __ldg(a.obs + src);
         if constexpr (kXYZ3) T[t] = __ldg(a.z + src);
     }
     __syncthreads();
-    // Panel 0 into cur: thread t takes column t mod 16, every (kT/16)-th row.
-    gen_column<kXYZ3>(cur, 0, X, Y, Z, T, M, Mp, 0, min(kNB, M), tid & 15, tid >> 4, kT >> 4, *mp);
-    __syncthreads();
+    KWindow kw{nullptr, a.ktab, 0};
+    if constexpr (GEN == kGenGeneral) {
+        // Largest possible squared distance: the bounding box's diagonal.
+        double x0 = X[0], x1 = x0, y0 = Y[0], y1 = y0;
+        for (int t = lane; t < M; t += 32) {
+            x0 = fmin(x0, X[t]);
+            x1 = fmax(x1, X[t]);
+            y0 = fmin(y0, Y[t]);
+            y1 = fmax(y1, Y[t]);
+        }
+#pragma unroll
+        for (int w = 16; w > 0; w >>= 1) {
+            x0 = fmin(x0, __shfl_xor_sync(0xffffffffu, x0, w));
+            x1 = fmax(x1, __shfl_xor_sync(0xffffffffu, x1, w));
+            y0 = fmin(y0, __shfl_xor_sync(0xffffffffu, y0, w));
+            y1 = fmax(y1, __shfl_xor_sync(0xffffffffu, y1, w));
+        }
+        const double dx = x1 - x0, dy = y1 - y0;
+        const int e = (__double2hiint(fma(dx, dx, dy * dy)) >> 20) + 1;  // exponent field above it
+        const int top = __ldg(&mp->kt_e1) + 1023;                        // of region 1's top
+        const int first = max(min(e, top) - kTabWinOct, top - kTabOct1);
+        unsigned dyn;
+        asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
+        if (__ldg(&mp->kt_on) && l.total + kTabWinBytes <= dyn) {
+            double2 *win = reinterpret_cast<double2 *>(smem + l.total);
+            const double2 *src = a.ktab + 8 * (first - (top - kTabOct1));
+            for (int t = tid; t < kTabPairs * kTabWinN; t += kT) {
+                const int h = t / kTabWinN;
+                win[t] = __ldg(src + h * kTabN + (t - h * kTabWinN));
+            }
+            kw.win = win;
+            kw.base = 8 * first;
+            __syncthreads();
+        }
+    }
 
-    unsigned st = 0;  // thread 0: pivot flags
-    for (int p = 0; p < P; ++p) {
-        const int k0 = p * kNB, kb = min(kNB, M - k0);
+    // Panel 0: thread t takes column t mod 16, every (kT/16)-th row; through
+    // the table, the update warps' code makes it (in nxt) before the first
+    // panel (for the closed forms that costs registers: C2's shape 3.17
+    // against 2.96 ms).
+    constexpr bool kFirst = GEN == kGenGeneral;
+    if constexpr (!kFirst) {
+        gen_column<kXYZ3>(cur, 0, X, Y, Z, T, M, Mp, 0, min(kNB, M), tid & 15, tid >> 4, kT >> 4, *mp);
+        __syncthreads();
+    }
+
+    unsigned st = 0;  // warp 0: pivot flags
+    for (int p = kFirst ? -1 : 0; p < P; ++p) {
+        const int k0 = kFirst ? max(0, p * kNB) : p * kNB;
+        const int kb = (kFirst && p < 0) ? 0 : min(kNB, M - k0);
         const int n0 = k0 + kb;                    // first row / column of panel p+1
         const int kb1 = max(0, min(kNB, M - n0));  // its width
         if (warp == 0) {
-            st |= factor_phase(cur, M, k0, kb, mc, sh);
+            if (!kFirst || p >= 0)
+                st |= factor_phase<(NT * MINB > 384)>(cur, M, k0, kb, mc, sh);
         } else if (kb1 > 0) {
-            if constexpr (GEN != kGenClosed) {
+            if constexpr (kXYZ3) {
                 const int u = tid - 32;
-                gen_column<kXYZ3>(nxt, n0, X, Y, Z, T, M, Mp, n0, kb1, u & 15, n0 + (u >> 4), (kT - 32) >> 4,
-                                  *mp);
+                gen_column<true>(nxt, n0, X, Y, Z, T, M, Mp, n0, kb1, u & 15, n0 + (u >> 4), (kT - 32) >> 4,
+                                 *mp);
                 update_warps_sync<NT>();
-                next_panel<false>(nxt, X, Y, Z, slab, M, p, n0, 1, kW - 1, mp);
+                next_panel<GEN>(nxt, X, Y, Z, slab, M, p, n0, 1, kW - 1, mp, kw);
             } else {
-                next_panel<true>(nxt, X, Y, Z, slab, M, p, n0, 1, kW - 1, mp);
+                next_panel<GEN>(nxt, X, Y, Z, slab, M, p, n0, 1, kW - 1, mp, kw);
             }
+        }
+        if (kFirst && p < 0) {
+            __syncthreads();
+            double *t = cur;
+            cur = nxt;
+            nxt = t;
+            continue;
         }
         // The substitution needs only the factored diagonal block: warp 0
         // publishes it (named barrier 3 over the CTA: warp 0 arrives, the

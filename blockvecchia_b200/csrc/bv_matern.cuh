@@ -54,6 +54,8 @@ struct MaternParams {
     double gam_p;       // Gamma(1 + mu)
     double gam_m;       // Gamma(1 - mu)
     double fact;        // pi mu / sin(pi mu)
+    // The table of the general-nu covariance (ktab_prepare, bv_ktab.cuh):
+    int kt_on, kt_e1;
 };
 
 // Host: the mu-only constants of the general-nu K_nu.  1/Gamma(1+z) by its

@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(NT, MINB) llh_lean_server_kernel(const JobDesc
                 a.block_status[b] = a.status_or;
             }
         } else {
-            process_block_lean<NT, GEN>(a, &d.mp, b, reinterpret_cast<unsigned char *>(smem), slab, sh);
+            process_block_lean<NT, MINB, GEN>(a, &d.mp, b, reinterpret_cast<unsigned char *>(smem), slab, sh);
         }
         __syncthreads();
         if (tid == 0) {
@@ -141,6 +141,15 @@ __global__ void __launch_bounds__(NT, MINB) llh_lean_server_kernel(const JobDesc
     }
 }
 
+// The general-nu tables of a batch's requests, one per grid row.
+__global__ void __launch_bounds__(kTabThreads) ktab_batch_kernel(const JobDesc *descs, double2 *tabs)
+{
+    const int idx = (int)(blockIdx.x * kTabThreads + threadIdx.x) >> 4;
+    const MaternParams &mp = descs[blockIdx.y].mp;
+    if (idx < kTabN && mp.nu_kind == kNuGeneral && mp.kt_on)
+        ktab_build_interval(mp, idx, tabs + (size_t)blockIdx.y * kTabEntries);
+}
+
 struct LeanServerVariant {
     void (*kernel[2])(const JobDesc *, const int2 *, int, unsigned *, double *, size_t);  // by LeanGen
     int threads;
@@ -150,6 +159,7 @@ struct LeanServerVariant {
 static const LeanServerVariant kLeanServer[] = {
     BV_LEAN_SERVER(96, 4),
     BV_LEAN_SERVER(128, 3),
+    BV_LEAN_SERVER(160, 2),
     BV_LEAN_SERVER(256, 2),
 };
 
@@ -237,6 +247,8 @@ struct bv_server {
         size_t cap_tasks = 0;
         JobDesc *desc = nullptr;
         EvalResult *res = nullptr;
+        double2 *ktab = nullptr;  // one general-nu table per request of the largest such batch
+        size_t cap_ktab = 0;
         unsigned *counters = nullptr;  // [0]: work counter, [1 + r]: request r's done count, then two work counters
         double *slab = nullptr;
         size_t slab_stride = 0;
@@ -277,6 +289,7 @@ struct bv_server {
     size_t smem_bytes = 0;
     int grid = 0;
     int lean_limit = 0;  // blocks up to this M run the streamed kernel
+    size_t lean_avail = 0;  // its largest dynamic shared memory
     int sms = 0;
     cudaStream_t upload = nullptr;
 };
@@ -347,6 +360,7 @@ void fill_params(MaternParams &p, const double *theta, double dist_scale)
     p.nugget = theta[3];
     p.model = kModel2D;
     matern_prepare(p);
+    ktab_prepare(p);
 }
 
 // Requests of admitted jobs are ready to run.
@@ -392,8 +406,8 @@ struct LeanLaunch {
 bool lean_launch_for(const bv_server *S, int gen, int max_m, size_t blocks, LeanLaunch &ll)
 {
     const int t = lean_table_threads(gen, max_m, blocks);
-    ll.v = &kLeanServer[t == 96 ? 0 : (t == 128 ? 1 : 2)];
-    ll.smem = std::max<size_t>(big_layout(max_m, 0, 0, 0).total, kReduceScratchBytes);
+    ll.v = &kLeanServer[t == 96 ? 0 : (t == 128 ? 1 : (t == 160 ? 2 : 3))];
+    ll.smem = std::max<size_t>(lean_smem(gen, max_m, 0, S->lean_avail), kReduceScratchBytes);
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ll.v->kernel[gen], ll.v->threads, ll.smem) != cudaSuccess ||
         occ < 1) {
@@ -497,6 +511,7 @@ bool launch_batch(bv_server *S, bv_server::Slot &sl, const std::vector<Job *> &j
         ll[g].grid = std::max(1, std::min<int>(ll[g].grid, (int)n_lean[g]));
         lean_bytes[g] = ll[g].stride * 8 * (size_t)ll[g].grid;
     }
+    if (ok && n_lean[kGenGeneral] > 0) ok = grow_async(sl.ktab, sl.cap_ktab, (size_t)R * kTabEntries, s);
     if (ok && lean_bytes[0] + lean_bytes[1] > sl.lean_bytes) {
         if (sl.lean_slab) cudaFreeAsync(sl.lean_slab, s);
         sl.lean_bytes = lean_bytes[0] + lean_bytes[1];
@@ -536,6 +551,7 @@ bool launch_batch(bv_server *S, bv_server::Slot &sl, const std::vector<Job *> &j
         a.big_max_m = j.big ? S->big_max_m : 0;
         a.log2pi = std::log(2 * 3.141592653589793);
         a.mp = nullptr;
+        a.ktab = gen[r] == kGenGeneral ? sl.ktab + (size_t)r * kTabEntries : nullptr;
         a.task_begin = a.task_end = 0;
         d.done = sl.counters + 1 + r;
         d.out = sl.res + r;
@@ -559,6 +575,7 @@ bool launch_batch(bv_server *S, bv_server::Slot &sl, const std::vector<Job *> &j
     for (int g = 0; ok && g < 2; ++g) {
         if (!ll[g].v) continue;
         cudaStream_t gs = (fork && g == 1) ? sl.s2 : s;
+        if (g == kGenGeneral) ktab_batch_kernel<<<dim3(kTabCtas, R), kTabThreads, 0, gs>>>(sl.desc, sl.ktab);
         ll[g].v->kernel[g]<<<ll[g].grid, ll[g].v->threads, ll[g].smem, gs>>>(
             sl.desc, sl.tasks + n_pers + (g ? n_lean[0] : 0), (int)n_lean[g], sl.counters + 1 + R + g,
             sl.lean_slab + (g ? lean_bytes[0] / 8 : 0), ll[g].stride);
@@ -721,6 +738,7 @@ void destroy_slot(bv_server::Slot &sl)
     cudaFree(sl.desc);
     cudaFree(sl.res);
     cudaFree(sl.counters);
+    cudaFree(sl.ktab);
     cudaFree(sl.slab);
     cudaFree(sl.lean_slab);
     cudaFreeHost(sl.h_tasks);
@@ -802,8 +820,9 @@ extern "C" int bv_server_create(const bv_server_opts *opts, bv_server **out)
     // The streamed kernel: the handles' limit, and its shared memory allowed.
     {
         cudaFuncAttributes fl;
-        BV_CUDA_TRY(cudaFuncGetAttributes(&fl, kLeanServer[2].kernel[kGenClosed]));
+        BV_CUDA_TRY(cudaFuncGetAttributes(&fl, kLeanServer[3].kernel[kGenClosed]));
         const size_t avail = (size_t)optin - fl.sharedSizeBytes;
+        S->lean_avail = avail;
         S->lean_limit = big_max_m_for_bytes(avail, 0, 0, 0);
         for (const LeanServerVariant &v : kLeanServer)
             for (auto k : v.kernel)

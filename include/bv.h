@@ -173,7 +173,8 @@ typedef struct {
     double tune_ms[6];   /* with bv_opts.tune: the streamed kernel's time on
                             the first evaluation per variant: 96 threads x 4
                             CTAs per SM, 160 x 3, 256 x 2, 128 x 3, 160 x 2
-                            and 256 x 1 (0 where not timed)                  */
+                            and 256 x 1 (with a third coordinate 96 x 5 and
+                            128 x 4; 0 where not timed)                      */
 } bv_status;
 
 typedef struct bv_handle bv_handle;

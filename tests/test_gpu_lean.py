@@ -56,8 +56,26 @@ def test_panel_edges(bvlib, oracle, cs):
     _check(bvlib, oracle, L, (0.7, 0.1, 1.5), dist_scale=2.0, nugget=0.05)
 
 
-@pytest.mark.parametrize("blocks", [590, 620])
+@pytest.mark.parametrize("blocks", [440, 450, 590, 600])
 def test_few_and_many_small_blocks(bvlib, oracle, blocks):
     """Both sides of the block count at which small blocks change CTA size."""
     L = _layout(bvlib, [40] + [1 + i % 9 for i in range(blocks - 1)], 30, seed=blocks)
     _check(bvlib, oracle, L, (1.0, 0.2, 0.5))
+
+
+@pytest.mark.parametrize("nu", [0.3, 0.8, 2.2])
+@pytest.mark.parametrize("range_", [1e-5, 0.003, 0.1, 30.0])
+def test_general_nu_table(bvlib, oracle, nu, range_):
+    """A general nu through the table: scaled distances within its regions,
+    below, between and beyond them (locations 1e-6 to 1.4 apart, ranges over
+    six decades), repeated locations, blocks smaller than a panel."""
+    g = np.random.default_rng(7)
+    L = _layout(bvlib, [33] + [1, 2, 5, 17, 30] * 4, 30, seed=3)
+    # Groups of points 1e-6, 1e-4 and 1e-2 apart around the first ones; the
+    # nugget keeps their covariances regular.
+    for k, h in enumerate((1e-6, 1e-4, 1e-2, 0.0)):
+        i = g.choice(L.n // 2, 12, replace=False)
+        L.x[L.n // 2 + 12 * k:L.n // 2 + 12 * (k + 1)] = L.x[i] + h * g.random(12)
+        L.y[L.n // 2 + 12 * k:L.n // 2 + 12 * (k + 1)] = L.y[i]
+    _check(bvlib, oracle, L, (1.1, range_, nu), nugget=0.1)
+    _check(bvlib, oracle, L, (1.1, range_ / 2, nu), dist_scale=2.0, nugget=0.1)
