@@ -22,6 +22,20 @@
 // whatever S member occupied position t moves to the winner's old position.
 // Members outside S never win and never change the relative positions of S
 // members, so the replay reproduces the reference's output, ties included.
+// When no two keys of S are equal the order is simply ascending, and each
+// member's rank is counted instead.
+//
+// Which candidates are streamed: planar and 3-D keys go through a uniform
+// grid over the locations (about four per cell, built on the device for the
+// call).  A block scans the cells of a square window around its centroid that
+// holds about 1.6 cs earlier points, keeps those with an index in its prefix,
+// and is done when its k-th pre-key is below the squared distance to the
+// window's nearest side -- no point outside can then belong to S; otherwise
+// the window grows.  Every key is computed from the same coordinates by the
+// same operations as in a scan of the whole prefix, and S does not depend on
+// the order of the candidates.  A scan of the whole prefix (5e10 keys at 1M
+// points and 100k blocks) remains for great-circle keys, small layouts and
+// prefixes, and windows that would hold more points than the prefix.
 // A block whose ties at the k-th key overflow the warp's buffer (hundreds of
 // exactly repeated locations at one distance) is listed and redone by
 // knn_heavy_kernel: one CTA, keys recomputed on every pass instead of
@@ -63,13 +77,174 @@ struct KnnArgs {
     unsigned *heavy_count;
     const int *list;  // blocks to select for (largest prefix first), or nullptr: all
     int nlist;
+    // The grid (ncell = 0: none): its shape, cell starts, and the locations in
+    // cell order with their indices.
+    const struct KnnGrid *grid;
+    const int *start;
+    const double *sx, *sy, *sz;
+    const int *sidx;
+    int n;
 };
+
+// Cells (cx, cy), row-major, of size hx x hy from (x0, y0).
+struct KnnGrid {
+    double x0, y0, hx, hy, ihx, ihy;
+    int nx, ny;
+};
+
+constexpr int kGridOcc = 4;         // mean locations per cell
+constexpr int kGridMinN = 4096;     // smaller layouts scan the prefix
+constexpr int kGridMinPrefix = 2048;  // and so do the first blocks of larger ones
+constexpr int kBoxCtas = 296, kBoxThreads = 256;
+
+__device__ __forceinline__ int grid_cell1(double v, double v0, double ih, int n)
+{
+    return min(max((int)((v - v0) * ih), 0), n - 1);
+}
+
+// Bounding box of the locations: partial boxes (x0, x1, y0, y1 per CTA) ...
+__global__ void __launch_bounds__(kBoxThreads) knn_box_kernel(const double *x, const double *y, int n,
+                                                             double *part)
+{
+    __shared__ double sh[4][kBoxThreads / 32];
+    double b[4] = {INFINITY, -INFINITY, INFINITY, -INFINITY};
+    for (int i = blockIdx.x * kBoxThreads + threadIdx.x; i < n; i += kBoxCtas * kBoxThreads) {
+        b[0] = fmin(b[0], x[i]);
+        b[1] = fmax(b[1], x[i]);
+        b[2] = fmin(b[2], y[i]);
+        b[3] = fmax(b[3], y[i]);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const double v = __shfl_xor_sync(0xffffffffu, b[k], o);
+            b[k] = (k & 1) ? fmax(b[k], v) : fmin(b[k], v);
+        }
+        if ((threadIdx.x & 31) == 0) sh[k][threadIdx.x >> 5] = b[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        const int k = threadIdx.x;
+        double v = sh[k][0];
+        for (int w = 1; w < kBoxThreads / 32; ++w) v = (k & 1) ? fmax(v, sh[k][w]) : fmin(v, sh[k][w]);
+        part[blockIdx.x * 4 + k] = v;
+    }
+}
+
+// ... and the grid's shape: square cells, at most ncell of them.
+__global__ void knn_grid_kernel(const double *part, int ncell, KnnGrid *grid)
+{
+    if (threadIdx.x != 0) return;
+    double b[4] = {part[0], part[1], part[2], part[3]};
+    for (int c = 1; c < kBoxCtas; ++c)
+        for (int k = 0; k < 4; ++k)
+            b[k] = (k & 1) ? fmax(b[k], part[4 * c + k]) : fmin(b[k], part[4 * c + k]);
+    KnnGrid g;
+    g.x0 = b[0];
+    g.y0 = b[2];
+    const double wx = b[1] - b[0], wy = b[3] - b[2];
+    // Sides without an extent (or not finite) get one column or row.
+    double nx = 1.0, ny = 1.0;
+    if (wx > 0.0 && wy > 0.0) {
+        nx = fmin(fmax(sqrt(ncell * (wx / wy)), 1.0), (double)ncell);
+        ny = fmax((double)ncell / nx, 1.0);
+    } else if (wx > 0.0) {
+        nx = ncell;
+    } else if (wy > 0.0) {
+        ny = ncell;
+    }
+    g.nx = max((int)nx, 1);
+    g.ny = max(min((int)ny, ncell / g.nx), 1);
+    g.hx = wx / g.nx;
+    g.hy = wy / g.ny;
+    g.ihx = (g.hx > 0.0 && isfinite(g.hx)) ? 1.0 / g.hx : 0.0;
+    g.ihy = (g.hy > 0.0 && isfinite(g.hy)) ? 1.0 / g.hy : 0.0;
+    *grid = g;
+}
+
+// Locations per cell (count), or their places in cell order (cursor).
+template <bool kScatter>
+__global__ void knn_cells_kernel(const double *x, const double *y, const double *z, int n,
+                                 const KnnGrid *grid, int *cells, double *sx, double *sy, double *sz,
+                                 int *sidx)
+{
+    const KnnGrid g = *grid;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const double px = x[i], py = y[i];
+        const int c = grid_cell1(py, g.y0, g.ihy, g.ny) * g.nx + grid_cell1(px, g.x0, g.ihx, g.nx);
+        const int p = atomicAdd(&cells[c], 1);
+        if constexpr (kScatter) {
+            sx[p] = px;
+            sy[p] = py;
+            if (z) sz[p] = z[i];
+            sidx[p] = i;
+        }
+    }
+}
+
+// Exclusive prefix sums of the counts by one CTA: start[0 .. ncell] and a copy
+// in the counts' place (the scatter's cursors).
+__global__ void __launch_bounds__(1024) knn_scan_kernel(int *count, int *start, int ncell)
+{
+    __shared__ int warp_sum[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int carry = 0;
+    for (int base = 0; base < ncell; base += 4096) {
+        int v[4], t = 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = base + tid * 4 + u;
+            v[u] = (i < ncell) ? count[i] : 0;
+            t += v[u];
+        }
+        int incl = t;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int w = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += w;
+        }
+        if (lane == 31) warp_sum[warp] = incl;
+        __syncthreads();
+        int before = carry, all = 0;
+        for (int w = 0; w < 32; ++w) {
+            if (w < warp) before += warp_sum[w];
+            all += warp_sum[w];
+        }
+        int run = before + incl - t;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = base + tid * 4 + u;
+            if (i < ncell) {
+                start[i] = run;
+                count[i] = run;
+            }
+            run += v[u];
+        }
+        carry += all;
+        __syncthreads();
+    }
+    if (tid == 0) start[ncell] = carry;
+}
 
 // Key geometries, each a separate instantiation: plane (2-D), 3-D (the
 // time_flag key), and the great-circle key of distance_metric = 1 (--earth,
 // include/nearest_neighbor.h:93-96: distanceEarth(centroid, point); z and cz
 // then carry cos(latitude) of the points and centroids, from the host).
 enum KnnGeo : int { kGeoPlane = 0, kGeo3D = 1, kGeoEarth = 2 };
+
+// The same for a planar or 3-D key from given coordinates.
+template <int kGeo>
+__device__ __forceinline__ double knn_prekey_at(double x, double y, double z, double cx, double cy, double cz)
+{
+    const double dx = x - cx;
+    const double dy = y - cy;
+    const double s = __fma_rn(dx, dx, __dmul_rn(dy, dy));
+    if constexpr (kGeo == kGeoPlane) return s;
+    const double d = __dsqrt_rn(s);
+    const double dz = cz - z;
+    return __fma_rn(d, d, __dmul_rn(dz, dz));
+}
 
 // The argument of the key's final square root for candidate p.
 template <int kGeo>
@@ -86,13 +261,8 @@ __device__ __forceinline__ double knn_prekey(const KnnArgs &a, int p, double cx,
         const double v = sin(__dmul_rn(__dsub_rn(lon2r, lon1r), 0.5));
         return __fma_rn(u, u, __dmul_rn(__dmul_rn(__dmul_rn(cz, __ldg(a.z + p)), v), v));
     }
-    const double dx = __ldg(a.x + p) - cx;
-    const double dy = __ldg(a.y + p) - cy;
-    const double s = __fma_rn(dx, dx, __dmul_rn(dy, dy));
-    if constexpr (kGeo == kGeoPlane) return s;
-    const double d = __dsqrt_rn(s);
-    const double dz = cz - __ldg(a.z + p);
-    return __fma_rn(d, d, __dmul_rn(dz, dz));
+    return knn_prekey_at<kGeo>(__ldg(a.x + p), __ldg(a.y + p), kGeo == kGeo3D ? __ldg(a.z + p) : 0.0, cx, cy,
+                               cz);
 }
 
 // The key (a distance) from its pre-key.
@@ -235,31 +405,20 @@ __global__ void __launch_bounds__(kKnnWarps * 32) knn_kernel(KnnArgs a)
             continue;
         }
 
-        // 1. Stream candidates 0..P-1 through the falling threshold.
+        // 1. Stream candidates through the falling threshold: the window of
+        // the grid around the centroid, or the whole prefix.
         unsigned long long lim = ~0ull;
         int count = 0;
         bool overflow = false;
-        for (int base = 0; base < P; base += 128) {
-            unsigned long long key[4];
-            bool keep[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int p = base + 32 * u + lane;
-                keep[u] = false;
-                key[u] = 0ull;
-                if (p < P) {
-                    const double s = knn_prekey<kGeo>(a, p, cx, cy, cz);
-                    key[u] = (unsigned long long)__double_as_longlong(s);
-                    keep[u] = key[u] <= lim;
-                }
-            }
+        // Four candidates per lane at a time; key[u] valid where keep[u].
+        auto take = [&](const unsigned long long (&key)[4], const bool (&keep)[4], const int (&id)[4]) {
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const unsigned bal = __ballot_sync(0xffffffffu, keep[u]);
                 if (keep[u]) {
                     const int p = count + __popc(bal & lanemask_lt());
                     w.key[p] = key[u];
-                    w.idx[p] = base + 32 * u + lane;
+                    w.idx[p] = id[u];
                 }
                 count += __popc(bal);
             }
@@ -268,10 +427,96 @@ __global__ void __launch_bounds__(kKnnWarps * 32) knn_kernel(KnnArgs a)
                 const unsigned long long kth = warp_kth(w, count, k);
                 lim = window_hi<kGeo>(kth);
                 count = warp_compact(w, count, lim);
-                if (count > kKnnCap - 128) {
-                    overflow = true;
+                if (count > kKnnCap - 128) overflow = true;
+            }
+        };
+        bool whole = true;
+        if (kGeo != kGeoEarth && a.grid && P >= kGridMinPrefix) {
+            const KnnGrid g = *a.grid;
+            const int gx = grid_cell1(cx, g.x0, g.ihx, g.nx), gy = grid_cell1(cy, g.y0, g.ihy, g.ny);
+            // Locations that should hold the set: 1.6 k earlier ones.
+            const double want = 1.6 * (double)k * ((double)a.n / (double)P);
+            int r = 1;
+            for (whole = false;;) {
+                // The smallest window (from the present one on) with as many.
+                int x0, x1, y0, y1, held;
+                for (;;) {
+                    x0 = max(gx - r, 0);
+                    x1 = min(gx + r, g.nx - 1);
+                    y0 = max(gy - r, 0);
+                    y1 = min(gy + r, g.ny - 1);
+                    held = 0;
+                    for (int row = y0 + lane; row <= y1; row += 32)
+                        held += a.start[row * g.nx + x1 + 1] - a.start[row * g.nx + x0];
+                    held = __reduce_add_sync(0xffffffffu, held);
+                    if ((double)held >= want || held >= P || held == a.n) break;
+                    r += (r + 2) / 3;
+                }
+                if (held >= P) {  // no fewer than the prefix: scan that
+                    whole = true;
                     break;
                 }
+                count = 0;
+                for (int row = y0; row <= y1 && !overflow; ++row) {
+                    const int j1 = a.start[row * g.nx + x1 + 1];
+                    for (int base = a.start[row * g.nx + x0]; base < j1 && !overflow; base += 128) {
+                        unsigned long long key[4];
+                        bool keep[4];
+                        int id[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const int j = base + 32 * u + lane;
+                            keep[u] = false;
+                            key[u] = 0ull;
+                            id[u] = 0;
+                            if (j < j1) {
+                                id[u] = a.sidx[j];
+                                const double s = knn_prekey_at<kGeo>(
+                                    a.sx[j], a.sy[j], kGeo == kGeo3D ? a.sz[j] : 0.0, cx, cy, cz);
+                                key[u] = (unsigned long long)__double_as_longlong(s);
+                                keep[u] = id[u] < P && key[u] <= lim;
+                            }
+                        }
+                        take(key, keep, id);
+                    }
+                }
+                if (overflow) break;
+                __syncwarp();
+                // Distance to the nearest side that has cells beyond it, less
+                // the rounding of the cell assignment.
+                double d = INFINITY;
+                if (x0 > 0) d = fmin(d, cx - (g.x0 + x0 * g.hx) - 1e-6 * g.hx);
+                if (x1 < g.nx - 1) d = fmin(d, (g.x0 + (x1 + 1) * g.hx) - cx - 1e-6 * g.hx);
+                if (y0 > 0) d = fmin(d, cy - (g.y0 + y0 * g.hy) - 1e-6 * g.hy);
+                if (y1 < g.ny - 1) d = fmin(d, (g.y0 + (y1 + 1) * g.hy) - cy - 1e-6 * g.hy);
+                if (count >= k) {
+                    const unsigned long long kth = warp_kth(w, count, k);
+                    lim = window_hi<kGeo>(kth);
+                    const double safe = d * (1.0 - 1e-9);
+                    if (d > 0.0 && __longlong_as_double((long long)lim) < safe * safe) break;
+                }
+                r += (r + 2) / 3;
+            }
+        }
+        if (whole) {
+            count = 0;
+            for (int base = 0; base < P && !overflow; base += 128) {
+                unsigned long long key[4];
+                bool keep[4];
+                int id[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int p = base + 32 * u + lane;
+                    id[u] = p;
+                    keep[u] = false;
+                    key[u] = 0ull;
+                    if (p < P) {
+                        const double s = knn_prekey<kGeo>(a, p, cx, cy, cz);
+                        key[u] = (unsigned long long)__double_as_longlong(s);
+                        keep[u] = key[u] <= lim;
+                    }
+                }
+                take(key, keep, id);
             }
         }
         if (overflow) {
@@ -314,7 +559,6 @@ __global__ void __launch_bounds__(kKnnWarps * 32) knn_kernel(KnnArgs a)
                     const int p = m + __popc(bal & lanemask_lt());
                     w.key[p] = (unsigned long long)__double_as_longlong(d);
                     w.idx[p] = id;
-                    w.pos[p] = id;  // initial position = index
                 }
                 m += __popc(bal);
                 __syncwarp();
@@ -322,7 +566,46 @@ __global__ void __launch_bounds__(kKnnWarps * 32) knn_kernel(KnnArgs a)
             count = m;
         }
 
-        // 3. Replay the selection sort on S.
+        // 3. Without equal keys in S (then |S| = k) the members in ascending
+        // order: each lane counts its members' ranks.
+        bool tie = count != k;
+        for (int j0 = 0; j0 < count && !tie; j0 += 32 * 4) {
+            unsigned long long kj[4];
+            int rank[4], same = 0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int j = j0 + 32 * u + lane;
+                kj[u] = (j < count) ? w.key[j] : ~0ull;
+                rank[u] = 0;
+            }
+            for (int t = 0; t < count; ++t) {
+                const unsigned long long kt = w.key[t];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    rank[u] += kt < kj[u] ? 1 : 0;
+                    same += kt == kj[u] ? 1 : 0;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int j = j0 + 32 * u + lane;
+                if (j < count) {
+                    same -= 1;  // itself
+                    w.pos[rank[u]] = w.idx[j];
+                }
+            }
+            tie = __any_sync(0xffffffffu, same > 0);
+        }
+        if (!tie) {
+            __syncwarp();
+            for (int t = lane; t < k; t += 32) out[t] = w.pos[t];
+            __syncwarp();
+            continue;
+        }
+        // Ties: replay the selection sort on S from the initial positions.
+        __syncwarp();
+        for (int j = lane; j < count; j += 32) w.pos[j] = w.idx[j];
+        __syncwarp();
         for (int t = 0; t < k; ++t) {
             unsigned long long bkey = ~0ull;
             int bpos = 0x7fffffff, bslot = -1, occ = -1;
@@ -557,6 +840,7 @@ int knn_device(const double *d_x, const double *d_y, const double *d_z, int n, i
     int *d_heavy = reinterpret_cast<int *>(d_counter + 3);
     int *d_list = d_heavy + bc;
     KnnHeavyScratch sc{nullptr, nullptr, nullptr};
+    double *d_grid = nullptr;
     do {
         if ((e = cudaMemcpyAsync(d_c, cx, sizeof(double) * bc, cudaMemcpyHostToDevice, s)) ||
             (e = cudaMemcpyAsync(d_c + bc, cy, sizeof(double) * bc, cudaMemcpyHostToDevice, s)) ||
@@ -586,6 +870,44 @@ int knn_device(const double *d_x, const double *d_y, const double *d_z, int n, i
         ka.heavy_count = d_heavy_count;
         ka.list = mask ? d_list : nullptr;
         ka.nlist = (int)list.size();
+        ka.grid = nullptr;
+        ka.n = n;
+        if (geo != kGeoEarth && n >= kGridMinN) {
+            // One scratch allocation: the locations in cell order, partial
+            // boxes, the grid, cell starts and counts, indices.
+            const int ncell = n / kGridOcc;
+            const size_t nd = (size_t)n * (d_z ? 3 : 2) + 4 * kBoxCtas + sizeof(KnnGrid) / sizeof(double) + 1;
+            const size_t ni = (size_t)n + 2 * (size_t)ncell + 1;
+            if ((e = cudaMalloc(&d_grid, nd * sizeof(double) + ni * sizeof(int)))) {
+                fail(e, "cudaMalloc (grid)");
+                break;
+            }
+            double *sx = d_grid, *sy = sx + n, *sz = sy + n;
+            double *part = d_z ? sz + n : sz;
+            KnnGrid *grid = reinterpret_cast<KnnGrid *>(part + 4 * kBoxCtas);
+            int *start = reinterpret_cast<int *>(d_grid + nd);
+            int *cells = start + ncell + 1, *sidx = cells + ncell;
+            if ((e = cudaMemsetAsync(cells, 0, sizeof(int) * (size_t)ncell, s))) {
+                fail(e, "memset");
+                break;
+            }
+            knn_box_kernel<<<kBoxCtas, kBoxThreads, 0, s>>>(d_x, d_y, n, part);
+            knn_grid_kernel<<<1, 32, 0, s>>>(part, ncell, grid);
+            const int gb = std::min((n + 255) / 256, 148 * 8);
+            knn_cells_kernel<false><<<gb, 256, 0, s>>>(d_x, d_y, d_z, n, grid, cells, sx, sy, sz, sidx);
+            knn_scan_kernel<<<1, 1024, 0, s>>>(cells, start, ncell);
+            knn_cells_kernel<true><<<gb, 256, 0, s>>>(d_x, d_y, d_z, n, grid, cells, sx, sy, sz, sidx);
+            if ((e = cudaGetLastError())) {
+                fail(e, "grid");
+                break;
+            }
+            ka.grid = grid;
+            ka.start = start;
+            ka.sx = sx;
+            ka.sy = sy;
+            ka.sz = sz;
+            ka.sidx = sidx;
+        }
         const size_t smem = sizeof(KnnWarpSmem) * kKnnWarps;
         if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem))) {
             fail(e, "attribute");
@@ -639,6 +961,7 @@ int knn_device(const double *d_x, const double *d_y, const double *d_z, int n, i
     } while (0);
     cudaFree(d_c);
     cudaFree(d_counter);
+    cudaFree(d_grid);
     cudaFree(sc.key);
     cudaFree(sc.idx);
     cudaFree(sc.pos);
