@@ -92,6 +92,31 @@ __global__ void __launch_bounds__(NT, MINB) llh_lean_kernel_t(LlhArgs a)
     }
 }
 
+// One warp per block (small blocks, 2-D closed forms); dynamic shared memory:
+// a.gslab_stride doubles per warp.
+__global__ void __launch_bounds__(kWarpThreads, 3) llh_warp_kernel(LlhArgs a)
+{
+    extern __shared__ __align__(128) double smem[];
+    __shared__ LeanShared sh[kWarpThreads / 32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int task_end = a.task_count ? min(a.task_end, *a.task_count) : a.task_end;
+    for (;;) {
+        int task = 0;
+        if (lane == 0) task = (int)atomicAdd(a.work_counter, 1u) + a.task_begin;
+        task = __shfl_sync(0xffffffffu, task, 0);
+        if (task >= task_end) break;
+        const int b = a.order[task];
+        if (a.acc[b + 1] == a.acc[b]) {  // empty block: contributes -(0 + 0 + 0) / 2
+            if (lane == 0) {
+                a.block_llk[b] = -0.0;
+                a.block_status[b] = a.status_or;
+            }
+        } else {
+            process_block_warp(a, a.mp, b, smem + warp * a.gslab_stride, sh[warp]);
+        }
+    }
+}
+
 struct LeanVariant {
     void (*kernel[3])(LlhArgs);  // by LeanGen
     int threads;
@@ -105,8 +130,13 @@ static const LeanVariant kLeanVariants[] = {
     BV_LEAN(128, 3, 4), BV_LEAN(160, 2, 2), BV_LEAN(256, 1, 1),
 };
 constexpr int kNumLean = (int)(sizeof(kLeanVariants) / sizeof(kLeanVariants[0]));
+// The last entry is the one-warp kernel where it applies (warp_variant).
+static bool warp_variant(int gen, int max_m) { return gen == kGenClosed && max_m <= kWarpMaxM; }
 static int lean_variant(int gen, int max_m, size_t blocks)
 {
+    // A launch that fills the SMs with warps; 500 blocks (cs = 20) take .017 ms
+    // on 96-thread CTAs and .021 one per warp.
+    if (warp_variant(gen, max_m) && blocks >= 4 * 148) return kNumLean - 1;
     const int t = lean_table_threads(gen, max_m, blocks);
     return t == 96 ? 0 : (t == 128 ? 3 : (t == 160 ? 4 : 2));
 }
@@ -187,12 +217,12 @@ struct bv_handle {
         int threads;
         int grid;
         size_t smem;
-        int variant;  // kLeanVariants index, -1: the persistent kernel
+        size_t stride;  // doubles of a CTA's slab (the one-warp kernel: of a warp's area)
+        int variant;    // kLeanVariants index, -1: the persistent kernel
     };
     struct Launch {
         int begin, end;
         double *slab;
-        size_t slab_stride;
         Kernel k[2];  // closed-form nu, general nu
     };
     std::vector<Launch> launches;
@@ -415,18 +445,25 @@ static int plan_lean_launch(bv_handle *h, const cudaDeviceProp &prop, int begin,
     h->lean_m = max_m;
     int optin = 0;
     BV_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
-    bv_handle::Launch ln{begin, end, nullptr, (big_slab_doubles(max_m) + 31) & ~(size_t)31, {}};
-    int grid = 0;
+    bv_handle::Launch ln{begin, end, nullptr, {}};
+    size_t slab = 0;
     for (int g = 0; g < 2; ++g) {
         bv_handle::Kernel &k = ln.k[g];
         const int gen = h->nz ? kGenXYZ : g;
         k.variant = h->lean_choice >= 0 ? h->lean_choice : lean_variant(gen, max_m, (size_t)(end - begin));
         const LeanVariant &v = kLeanVariants[k.variant];
-        k.fn = v.kernel[gen];
-        k.threads = v.threads;
+        const bool warp = k.variant == kNumLean - 1 && warp_variant(gen, max_m);
+        k.fn = warp ? llh_warp_kernel : v.kernel[gen];
+        k.threads = warp ? kWarpThreads : v.threads;
         cudaFuncAttributes fa;
         BV_CUDA_TRY(cudaFuncGetAttributes(&fa, k.fn));
         k.smem = lean_smem(gen, max_m, h->nz, (size_t)optin - fa.sharedSizeBytes);
+        k.stride = (big_slab_doubles(max_m) + 31) & ~(size_t)31;
+        const int per = warp ? kWarpThreads / 32 : 1;  // blocks of a CTA at a time
+        if (warp) {
+            k.stride = warp_area_doubles(max_m);
+            k.smem = per * k.stride * sizeof(double);
+        }
         if (k.smem > (size_t)optin - fa.sharedSizeBytes) {
             set_error("plan: blocks of M = %d exceed the streamed schedule's shared memory", max_m);
             return BV_E_TOOLARGE;
@@ -436,16 +473,16 @@ static int plan_lean_launch(bv_handle *h, const cudaDeviceProp &prop, int begin,
         BV_CUDA_TRY(cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)((size_t)optin - fa.sharedSizeBytes)));
         int occ = 0;
-        BV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k.fn, v.threads, k.smem));
+        BV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k.fn, k.threads, k.smem));
         if (occ < 1) {
             set_error("plan: streamed kernel cannot be resident (smem %zu B)", k.smem);
             return BV_E_TOOLARGE;
         }
-        k.grid = std::min(prop.multiProcessorCount * occ, end - begin);
-        grid = std::max(grid, k.grid);
+        k.grid = std::min(prop.multiProcessorCount * occ, (end - begin + per - 1) / per);
+        if (!warp) slab = std::max(slab, k.stride * (size_t)k.grid);
     }
-    const size_t bytes = ln.slab_stride * sizeof(double) * (size_t)grid;
-    if (cudaMalloc(&h->d_slab_lean, bytes) != cudaSuccess) {
+    const size_t bytes = slab * sizeof(double);
+    if (bytes > 0 && cudaMalloc(&h->d_slab_lean, bytes) != cudaSuccess) {
         cudaGetLastError();
         set_error("plan: cannot allocate %zu B of block slabs", bytes);
         return BV_E_NOMEM;
@@ -534,8 +571,8 @@ static int plan_launches(bv_handle *h)
         }
     }
     auto persistent = [&](int begin, int end, int grid) {
-        const bv_handle::Kernel k{h->kernel, kThreads, grid, h->smem_bytes, -1};
-        h->launches.push_back({begin, end, h->d_slab, h->slab_stride, {k, k}});
+        const bv_handle::Kernel k{h->kernel, kThreads, grid, h->smem_bytes, h->slab_stride, -1};
+        h->launches.push_back({begin, end, h->d_slab, {k, k}});
     };
     if (sched != BV_SCHED_BUCKETED) {
         if (split > 0)
@@ -658,7 +695,7 @@ static int enqueue_eval(bv_handle *h, cudaStream_t s, int kind)
             a.task_count = h->mixed.fallback_count;
             a.status_or = BV_ST_FP32_FALLBACK;
             a.gslab = ln.slab;
-            a.gslab_stride = ln.slab_stride;
+            a.gslab_stride = ln.k[kind].stride;
             ln.k[kind].fn<<<ln.k[kind].grid, ln.k[kind].threads, ln.k[kind].smem, s>>>(a);
             BV_CUDA_TRY(cudaGetLastError());
         } else if (h->owned > 0) {
@@ -673,7 +710,7 @@ static int enqueue_eval(bv_handle *h, cudaStream_t s, int kind)
             const bv_handle::Launch &ln = h->launches[l];
             LlhArgs a = fp64_args(h->d_counters + l, h->d_order, ln.begin, ln.end);
             a.gslab = ln.slab;
-            a.gslab_stride = ln.slab_stride;
+            a.gslab_stride = ln.k[kind].stride;
             ln.k[kind].fn<<<ln.k[kind].grid, ln.k[kind].threads, ln.k[kind].smem, s>>>(a);
             BV_CUDA_TRY(cudaGetLastError());
         }

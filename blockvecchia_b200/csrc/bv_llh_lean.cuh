@@ -94,7 +94,7 @@ struct alignas(16) LeanShared {
     double Lt[kNB][kNB];  // factored diagonal block, transposed
     double inv[kNB];      // 1 / L_jj (0: failed pivot)
     double ex[4][8];      // factor_panel's exchange of a 4 x 4 diagonal block
-    double red[2][8];     // per-warp sums (at most 8 warps)
+    double red[2];        // the server's flag between blocks
     unsigned status;
     int task;
 };
@@ -294,7 +294,8 @@ __device__ __forceinline__ void gen_tiles_table(double (&d)[NTILE][2][2], const 
 // this SM.  Rows beyond the block read the following panel's memory (panel
 // q + 1 holds at least 18 rows whenever panel q is applied); they only reach
 // rows and columns that are never stored or never used.
-template <int NTILE>
+// kShared: the panels are in shared memory (the one-warp kernel).
+template <int NTILE, bool kShared>
 struct Frags {
     double2 b[2][2], a[NTILE][2];
     __device__ __forceinline__ void load(const double *pb, const double *pa, int tstep, const TileLane &L)
@@ -306,8 +307,8 @@ struct Frags {
         }
 #pragma unroll
         for (int m = 0; m < NTILE; ++m) {
-            a[m][0] = ldcg2(pa + m * tstep + L.o0);
-            a[m][1] = ldcg2(pa + m * tstep + L.o1);
+            a[m][0] = kShared ? ld2(pa + m * tstep + L.o0) : ldcg2(pa + m * tstep + L.o0);
+            a[m][1] = kShared ? ld2(pa + m * tstep + L.o1) : ldcg2(pa + m * tstep + L.o1);
         }
     }
     // A lane's DMMA steps 2h and 2h+1 use the adjacent columns k = 8h + 2 c4
@@ -328,7 +329,7 @@ struct Frags {
 // NTILE tiles (first tile at row i0, the others rstep rows further each) take
 // panels 0..p-1 from the slab.  Row i of panel q is at slab + 16 (q (Mp - 8q
 // - 8) + i).
-template <int NTILE>
+template <int NTILE, bool kShared = false>
 __device__ __forceinline__ void update_tiles(double (&d)[NTILE][2][2], const double *slab, int Mp, int p,
                                              int n0, int i0, int rstep, const TileLane &L)
 {
@@ -336,7 +337,7 @@ __device__ __forceinline__ void update_tiles(double (&d)[NTILE][2][2], const dou
     const double *pb = slab + 16 * (n0 + L.r8), *pa = slab + 16 * (i0 + L.r8);
     const int tstep = 16 * rstep;
     int step = 16 * (Mp - 16);  // from panel q to q + 1
-    Frags<NTILE> f0, f1;
+    Frags<NTILE, kShared> f0, f1;
     f0.load(pb, pa, tstep, L);
     for (int q = 0; q < p; q += 2) {
         if (q + 1 < p) {
@@ -688,6 +689,52 @@ __device__ __forceinline__ void solve_row(const LeanShared &sh, double *row, int
     store_row(row, r, w);
 }
 
+// log det of the conditional factor (positive pivots) and |u|^2 (row M) of the
+// finished panels: one sum per 32 columns, by warps 0 .. kW-1 in turn, into
+// sh.Lt (free by then); publish_block adds them in column order, so the value
+// does not depend on the number of warps.
+template <int kW>
+__device__ __forceinline__ void column_sums(const double *slab, int M, int mc, int warp, LeanShared &sh)
+{
+    const int lane = threadIdx.x & 31, Mp = M + 1;
+    for (int c = warp; mc + 32 * c < M; c += kW) {
+        const int j = mc + 32 * c + lane;
+        double ld = 0.0, qf = 0.0;
+        if (j < M) {
+            const int q = j / kNB, cc = j - q * kNB;
+            const double *pq = slab + big_panel_base(q, Mp);
+            const double dj = pq[(j - q * kNB) * 16 + swz(j, cc)];
+            if (dj > 0) ld = log(dj * dj);
+            const double u = pq[(M - q * kNB) * 16 + swz(M, cc)];
+            qf = u * u;
+        }
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1) {
+            ld += __shfl_xor_sync(0xffffffffu, ld, s);
+            qf += __shfl_xor_sync(0xffffffffu, qf, s);
+        }
+        if (lane == 0) {
+            (&sh.Lt[0][0])[c] = ld;
+            (&sh.Lt[8][0])[c] = qf;
+        }
+    }
+}
+
+// The block's contribution and status (one thread, after column_sums).
+__device__ __forceinline__ void publish_block(const LlhArgs &a, int b, int bs, const LeanShared &sh,
+                                              unsigned status)
+{
+    double Ls = 0.0, Qs = 0.0;
+    for (int c = 0; 32 * c < bs; ++c) {
+        Ls += (&sh.Lt[0][0])[c];
+        Qs += (&sh.Lt[8][0])[c];
+    }
+    const double v = -(Qs + Ls + (double)bs * a.log2pi) * 0.5;
+    if (!isfinite(v)) status |= BV_ST_NONFINITE;
+    a.block_llk[b] = v;
+    a.block_status[b] = status | a.status_or;
+}
+
 // One block by the streamed path, run by a CTA of NT threads (warp 0 factors
 // and solves, the other NT/32 - 1 warps generate and update).  smem: the
 // dynamic area (big_layout(M, 0, nz, 0).total bytes); slab: this CTA's global
@@ -831,39 +878,131 @@ __device__ __forceinline__ void process_block_lean(const LlhArgs &a, const Mater
         nxt = t;
     }
 
-    // log det of the conditional factor (positive pivots) and |u|^2 (row M).
-    double ld = 0.0, qf = 0.0;
-    for (int j = mc + tid; j < M; j += kT) {
-        const int q = j / kNB, c = j - q * kNB;
-        const double *pq = slab + big_panel_base(q, Mp);
-        const double dj = pq[(j - q * kNB) * 16 + swz(j, c)];
-        if (dj > 0) ld += log(dj * dj);
-        const double u = pq[(M - q * kNB) * 16 + swz(M, c)];
-        qf = fma(u, u, qf);
-    }
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) {
-        ld += __shfl_xor_sync(0xffffffffu, ld, s);
-        qf += __shfl_xor_sync(0xffffffffu, qf, s);
-    }
-    if (lane == 0) {
-        sh.red[0][warp] = ld;
-        sh.red[1][warp] = qf;
-    }
+    column_sums<kW>(slab, M, mc, warp, sh);
     if (warp == 0 && lane == 0 && st) atomicOr(&sh.status, st);
     __syncthreads();
     if (tid == 0) {
-        double Ls = 0.0, Qs = 0.0;
-        for (int w = 0; w < kW; ++w) {
-            Ls += sh.red[0][w];
-            Qs += sh.red[1][w];
-        }
-        const double v = -(Qs + Ls + (double)bs * a.log2pi) * 0.5;
-        unsigned s2 = sh.status;
-        if (!isfinite(v)) s2 |= BV_ST_NONFINITE;
-        a.block_llk[b] = v;
-        a.block_status[b] = s2 | a.status_or;
+        publish_block(a, b, bs, sh, sh.status);
     }
+}
+
+
+// ---------------------------------------------------------------------------
+// Small blocks: one warp per block.
+//
+// With M below ~50 a block has two or three panels of a few tiles each: the
+// streamed kernel's CTA spends its time in barriers and on one warp's pivot
+// chain while the others wait.  Here each warp works on a block of its own,
+// with all its panels in shared memory (no slab, no copy, no block-wide
+// barrier), so an SM overlaps the chains of 12 blocks instead of four.  The
+// operations per element and their order are the streamed kernel's.  Kernel
+// ms, 96-thread CTAs / one warp per block: classic, 30k blocks, cs = 30: 0.57
+// / 0.32; cs = 10, 20k: 0.23 / 0.11; cs = 47, 30k: 0.89 / 0.61; 5k blocks of 4
+// points, cs = 20: .099 / .058.  168 registers without spills (16 warps per SM
+// at 128: 0.30-0.43).
+// ---------------------------------------------------------------------------
+
+constexpr int kWarpMaxM = 48;   // largest block (three panels)
+constexpr int kWarpThreads = 128;
+
+// Doubles of a warp's area: X, Y, Z padded to whole panels, then the panels
+// and 16 rows of slack (a tile's rows beyond the block are read, not used).
+__host__ __device__ inline size_t warp_area_doubles(int M)
+{
+    return (3 * 16 * (size_t)big_panels(M) + big_slab_doubles(M) + 256 + 15) & ~(size_t)15;
+}
+
+// Tiles t0, t0 + 1 (NTILE = 2) or t0 of panel p+1 (rows n0..): generated,
+// panels 0..p applied, in place in the slab.
+template <int NTILE>
+__device__ __forceinline__ void warp_tiles(const double *X, const double *Y, const double *Z, double *slab,
+                                           int M, int p, int n0, int t0, const TileLane &L,
+                                           const MaternParams *mp)
+{
+    const int Mp = M + 1, i0 = n0 + 8 * t0;
+    double d[NTILE][2][2];
+    gen_tiles<NTILE>(d, X, Y, Z, M, n0, i0, 8, L, mp);
+    update_tiles<NTILE, true>(d, slab, Mp, p, n0, i0, 8, L);
+    double acc[NTILE][2][2];
+#pragma unroll
+    for (int m = 0; m < NTILE; ++m)
+#pragma unroll
+        for (int nj = 0; nj < 2; ++nj) acc[m][nj][0] = acc[m][nj][1] = 0.0;
+    if (p >= 0) {
+        // Panel p's products, summed from zero and subtracted.
+        const double *cur = slab + 16 * (p * (Mp - 8 * p - 8)) + 16 * L.r8 + L.c4;
+        const int x = (L.r8 & 3) << 2;
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+            const int k = (4 * kk) ^ x;
+            const double b0 = cur[16 * n0 + k], b1 = cur[16 * (n0 + 8) + k];
+#pragma unroll
+            for (int m = 0; m < NTILE; ++m) {
+                const double a = cur[16 * (i0 + 8 * m) + k];
+                dmma_8x8x4(acc[m][0][0], acc[m][0][1], a, b0);
+                dmma_8x8x4(acc[m][1][0], acc[m][1][1], a, b1);
+            }
+        }
+    }
+    double *nxt = slab + big_panel_base(p + 1, Mp);
+#pragma unroll
+    for (int m = 0; m < NTILE; ++m) {
+        const int i = i0 + 8 * m + L.r8;
+        if (i < Mp) {
+            double *row = nxt + 16 * (i - n0);
+            *reinterpret_cast<double2 *>(row + L.o0) =
+                make_double2(-d[m][0][0] - acc[m][0][0], -d[m][0][1] - acc[m][0][1]);
+            *reinterpret_cast<double2 *>(row + L.o1) =
+                make_double2(-d[m][1][0] - acc[m][1][0], -d[m][1][1] - acc[m][1][1]);
+        }
+    }
+}
+
+// One block (2-D, closed forms) by one warp; area: warp_area_doubles(M).
+__device__ __forceinline__ void process_block_warp(const LlhArgs &a, const MaternParams *mp, int b, double *area,
+                                                   LeanShared &sh)
+{
+    const int lane = threadIdx.x & 31;
+    const int off = a.acc[b];
+    const int bs = a.acc[b + 1] - off;
+    const int mc = (b == 0) ? 0 : a.cs;
+    const int M = mc + bs, Mp = M + 1, P = big_panels(M);
+    double *X = area, *Y = X + 16 * P, *Z = Y + 16 * P, *slab = Z + 16 * P;
+    const int *kidx = a.knn + (size_t)b * a.cs;
+    for (int t = lane; t < M; t += 32) {
+        const int src = (t < mc) ? __ldg(kidx + t) : off + (t - mc);
+        X[t] = __ldg(a.x + src);
+        Y[t] = __ldg(a.y + src);
+        Z[t] = __ldg(a.obs + src);
+    }
+    __syncwarp();
+    const TileLane L;
+    unsigned st = 0;
+    for (int p = -1; p < P; ++p) {
+        const int k0 = max(0, p * kNB), kb = (p < 0) ? 0 : min(kNB, M - k0), n0 = k0 + kb;
+        if (p >= 0) {
+            double *cur = slab + big_panel_base(p, Mp);
+            st |= factor_phase<false>(cur, M, k0, kb, mc, sh);
+            __syncwarp();
+            for (int r = k0 + (kb == kNB ? 2 * kNB : kb) + lane; r < Mp; r += 32)
+                solve_row(sh, cur + (r - k0) * 16, r);
+            __syncwarp();
+        }
+        if (n0 < M) {
+            const int ntiles = (Mp - n0 + 7) >> 3;
+            for (int t0 = 0; t0 < ntiles; t0 += 2) {
+                if (t0 + 1 < ntiles)
+                    warp_tiles<2>(X, Y, Z, slab, M, p, n0, t0, L, mp);
+                else
+                    warp_tiles<1>(X, Y, Z, slab, M, p, n0, t0, L, mp);
+            }
+            __syncwarp();
+        }
+    }
+    column_sums<1>(slab, M, mc, 0, sh);
+    __syncwarp();
+    if (lane == 0) publish_block(a, b, bs, sh, st);
+    __syncwarp();
 }
 
 }  // namespace bv

@@ -131,10 +131,10 @@ __global__ void __launch_bounds__(NT, MINB) llh_lean_server_kernel(const JobDesc
         if (tid == 0) {
             __threadfence();
             const unsigned prev = atomicAdd(d.done, 1u);
-            sh.red[0][0] = (prev + 1u == (unsigned)a.bc) ? 1.0 : 0.0;
+            sh.red[0] = (prev + 1u == (unsigned)a.bc) ? 1.0 : 0.0;
         }
         __syncthreads();
-        if (sh.red[0][0] != 0.0) {
+        if (sh.red[0] != 0.0) {
             __threadfence();
             reduce_blocks(a.block_llk, a.block_status, a.bc, d.out, smem);
         }

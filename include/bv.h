@@ -174,7 +174,9 @@ typedef struct {
                             the first evaluation per variant: 96 threads x 4
                             CTAs per SM, 160 x 3, 256 x 2, 128 x 3, 160 x 2
                             and 256 x 1 (with a third coordinate 96 x 5 and
-                            128 x 4; 0 where not timed)                      */
+                            128 x 4; blocks up to M = 48 at a closed-form nu
+                            one per warp in the last's place; 0 where not
+                            timed)                                           */
 } bv_status;
 
 typedef struct bv_handle bv_handle;

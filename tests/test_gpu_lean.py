@@ -63,6 +63,22 @@ def test_few_and_many_small_blocks(bvlib, oracle, blocks):
     _check(bvlib, oracle, L, (1.0, 0.2, 0.5))
 
 
+@pytest.mark.parametrize("cs", [0, 1, 14, 15, 16, 31])
+@pytest.mark.parametrize("nu", [0.5, 1.5, 2.5])
+def test_one_warp_per_block(bvlib, oracle, cs, nu):
+    """Launches of small blocks (M <= 48), one block per warp: every size up to
+    three full panels, empty blocks between, and the bits of a launch of few
+    blocks (CTAs per block)."""
+    top = 48 - cs
+    L = _layout(bvlib, [max(cs, 20)] + [1 + i % top for i in range(640)] + [0, 3, 0], cs, seed=cs)
+    _check(bvlib, oracle, L, (1.1, 0.15, nu), nugget=0.02)
+    th = (1.1, 0.15, nu, 0.02)
+    with bvlib.LlhData(L, nugget=True) as D, bvlib.LlhData(L, nugget=True, shard_count=3) as S:
+        D(th), S(th)
+        mine = bvlib.shard_blocks(L.batchNum, cs, 3, 0)
+        assert np.array_equal(D.block_llk()[mine], S.block_llk()[mine])
+
+
 @pytest.mark.parametrize("nu", [0.3, 0.8, 2.2])
 @pytest.mark.parametrize("range_", [1e-5, 0.003, 0.1, 30.0])
 def test_general_nu_table(bvlib, oracle, nu, range_):
