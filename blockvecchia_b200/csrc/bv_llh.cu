@@ -121,24 +121,23 @@ struct LeanVariant {
     void (*kernel[3])(LlhArgs);  // by LeanGen
     int threads;
 };
-#define BV_LEAN(NT, MINB, MINB3)                                                                   \
+#define BV_LEAN(NT, MINB)                                                                          \
     {{llh_lean_kernel_t<NT, MINB, kGenClosed>, llh_lean_kernel_t<NT, MINB, kGenGeneral>,          \
-      llh_lean_kernel_t<NT, MINB3, kGenXYZ>}, NT}
-// The table's four and two others (lean_table_threads has the measurements).  All give the same bits, so bv_opts.tune may pick any.
+      llh_lean_kernel_t<NT, MINB, kGenXYZ>}, NT}
+// In the order of LeanShape, and one more for the tuner; the last entry is the
+// one-warp kernel where it applies (warp_variant).  All give the same bits, so
+// bv_opts.tune may pick any.
 static const LeanVariant kLeanVariants[] = {
-    BV_LEAN(96, 4, 5),  BV_LEAN(160, 3, 3), BV_LEAN(256, 2, 2),
-    BV_LEAN(128, 3, 4), BV_LEAN(160, 2, 2), BV_LEAN(256, 1, 1),
+    BV_LEAN(96, 5), BV_LEAN(160, 3), BV_LEAN(256, 2), BV_LEAN(128, 4), BV_LEAN(160, 2), BV_LEAN(256, 1),
 };
 constexpr int kNumLean = (int)(sizeof(kLeanVariants) / sizeof(kLeanVariants[0]));
-// The last entry is the one-warp kernel where it applies (warp_variant).
 static bool warp_variant(int gen, int max_m) { return gen == kGenClosed && max_m <= kWarpMaxM; }
 static int lean_variant(int gen, int max_m, size_t blocks)
 {
     // A launch that fills the SMs with warps; 500 blocks (cs = 20) take .017 ms
     // on 96-thread CTAs and .021 one per warp.
     if (warp_variant(gen, max_m) && blocks >= 4 * 148) return kNumLean - 1;
-    const int t = lean_table_threads(gen, max_m, blocks);
-    return t == 96 ? 0 : (t == 128 ? 3 : (t == 160 ? 4 : 2));
+    return lean_table(gen, max_m, blocks);
 }
 
 __global__ void __launch_bounds__(kTabThreads) ktab_kernel(const MaternParams *mp, double2 *tab)

@@ -5,13 +5,17 @@
 //
 // Per 16-column panel p, warp 0 factors panel p's diagonal block and solves
 // the rows below it while the other warps bring panel p+1 up to date.  An
-// update warp owns groups of kDT tiles of 8 rows x 16 columns of panel p+1
-// and keeps a group's entries in the DMMA accumulators from their generation
-// to their last update from the slab:
+// update warp takes tiles of 8 rows x 16 columns of panel p+1 and keeps a
+// tile's entries in the DMMA accumulators from their generation to their last
+// update from the slab:
 //   * the lane that holds entry (i, j) in the m8n8k4 accumulator layout
-//     evaluates its covariance (4 kDT independent entries per lane, so the
+//     evaluates its covariance (four independent entries per lane, so the
 //     square-root and exponential chains overlap) -- the panel never makes
-//     the round trip through shared memory between generation and update;
+//     the round trip through shared memory between generation and update.
+//     One tile at a time: two at once, with eight entries in flight, ran n =
+//     1M, cs = 200 in 44.3 ms against 34.8 -- their unrolled code overflowed
+//     the instruction cache (13% of the warps' stall cycles) and 128
+//     registers;
 //   * panels 0..p-1 are applied straight from the CTA's slab (L2-resident),
 //     the next panel's fragments loaded while the current one is applied.
 //     The accumulators hold the entries negated, so D = A B + D subtracts
@@ -45,47 +49,49 @@ inline size_t lean_smem(int gen, int max_m, int nz, size_t avail)
     return gen == kGenGeneral ? std::max(b, std::min(avail, b + kTabWinBytes)) : b;
 }
 
-// CTA size of the streamed kernel for a launch of `blocks` blocks, the largest
-// of M = max_m (the handles and the server use it).  128 threads keep warp 0,
-// whose pivot chain is the block's critical path, on an SM sub-partition
-// without update warps: a warp issuing FP64 MMAs back to back beside the
-// chain stretched it from 5.2k to 16.9k cycles per panel.  Below M ~ 115 the
-// panels leave an update warp too few tiles, and 96 threads with four CTAs
-// per SM win; a launch of at most one wave of 128-thread CTAs wants each
-// block short instead, and one that 96-thread CTAs finish in one wave takes
-// those.  Beyond M ~ 240 only two CTAs' panels fit an SM: 160 threads without
-// spills, or 256 where few waves of blocks make the last one count.  Entries
-// generated through shared memory (a third coordinate) are a larger share of
-// the update warps' work: more of them.  Kernel ms at 96 x 4 CTAs per SM /
-// 160 x 3 / 256 x 2 / 128 x 3 / 160 x 2:
-//   cs =  30, classic, 30k blocks (M <=  31): 0.55 / 0.94 / 1.30 / 0.66 / 0.96
-//   cs =  60, 150 blocks (M <=  82):          .042 / .047 / .045 / .036 / .037
-//   cs =  60, 5k blocks (M <=  77):           0.27 / 0.42 / 0.55 / 0.30 / 0.39
-//   cs =  80, 10k blocks (M <=  97):          0.77 / 1.13 / 1.44 / 0.80 / 1.01
-//   cs = 120, 20k blocks (M <= 137):          3.15 / 3.88 / 4.63 / 2.96 / 3.48
-//   cs = 160, 10k blocks (M <= 177):          2.74 / 3.20 / 3.40 / 2.66 / 2.85
-//   cs = 200, 100k blocks (M <= 217):         53.1 / 50.9 / 48.8 / 44.0 / 45.5
-//   cs = 240, 10k blocks (M <= 257):          7.29 / 6.96 / 6.68 / 6.19 / 6.09
-//   cs = 300, 1.5k blocks (M <= 322):         2.68 / 1.89 / 1.64 / 1.96 / 1.76
-//   cs = 300, 20k blocks (M <= 317):          30.9 / 21.7 / 20.8 / 22.8 / 19.7
-//   nu = 0.8, cs =  80, 10k (M <=  97):       1.07 / 1.44 / 1.74 / 1.11 / 1.35
-//   nu = 0.8, cs = 120, 10k (M <= 137):       2.11 / 2.64 / 2.87 / 2.03 / 2.36
-//   nu = 0.8, cs = 200, 10k (M <= 217):       5.55 / 7.00 / 6.32 / 4.86 / 5.38
-//   nu = 0.8, cs = 300, 20k (M <= 317):       34.1 / 32.7 / 27.2 / 26.1 / 25.1
-// and for a third coordinate at 96 x 5 / 160 x 3 / 256 x 2 / 128 x 4 / 160 x 2:
-//   cs =  30, 2.5k blocks (M <=  44):         0.21 / 0.22 / 0.27 / 0.21 / 0.27
-//   cs =  47, 250 blocks (M <=  61):          .103 / .065 / .058 / .077 / .062
-//   cs =  60, 500 blocks (M <=  74):          .144 / .144 / .129 / .124 / .142
-//   cs =  60, 2.5k blocks (M <=  74):         0.53 / 0.48 / 0.51 / 0.49 / 0.60
-//   cs = 100, 2.5k blocks (M <= 114):         1.13 / 0.98 / 0.98 / 1.02 / 1.28
-//   cs = 200, 2.5k blocks (M <= 214):         5.40 / 3.24 / 3.07 / 3.98 / 4.30
-inline int lean_table_threads(int gen, int max_m, size_t blocks)
+// Variants of the streamed kernel, threads x CTAs per SM (the handles' and the
+// server's kernel arrays begin with these): 128 registers per thread, 204 for
+// the last.
+enum LeanShape : int { kLean96 = 0, kLean160 = 1, kLean256 = 2, kLean128 = 3, kLean160Wide = 4, kLeanShapes = 5 };
+
+// The variant for a launch of `blocks` blocks, the largest of M = max_m.  More
+// and larger CTAs per SM as long as two panels per CTA fit its shared memory:
+// four up to M ~ 185, three up to ~ 250, two beyond; a panel of a small block
+// has too few tiles for more than two update warps; a launch of at most two
+// blocks per SM wants each block short.  Entries generated through shared
+// memory (a third coordinate) are a larger share of the update warps' work.
+// Kernel ms at 96 x 5 / 160 x 3 / 256 x 2 / 128 x 4 / 160 x 2:
+//   cs =  60, 150 blocks (M <=  82):    .041 / .035 / .033 / .037 / .032
+//   cs = 120, 300 blocks (M <= 137):    .086 / .064 / .064 / .070 / .061
+//   cs = 120, 500 blocks (M <= 137):    .099 / .107 / .109 / .092 / .107
+//   cs =  60, 5k blocks (M <=  77):     0.25 / 0.31 / 0.42 / 0.27 / 0.38
+//   cs =  80, 10k blocks (M <=  97):    0.74 / 0.81 / 1.08 / 0.73 / 1.01
+//   cs = 120, 20k blocks (M <= 137):    2.91 / 2.83 / 3.37 / 2.67 / 3.34
+//   cs = 160, 10k blocks (M <= 177):    2.59 / 2.33 / 2.58 / 2.22 / 2.76
+//   cs = 200, 100k blocks (M <= 217):   47.5 / 34.7 / 37.4 / 37.8 / 42.9
+//   cs = 240, 10k blocks (M <= 257):    7.28 / 5.21 / 5.26 / 5.77 / 6.25
+//   cs = 300, 1.5k blocks (M <= 322):   2.91 / 1.87 / 1.45 / 2.09 / 1.86
+//   cs = 300, 20k blocks (M <= 317):    33.4 / 20.9 / 17.1 / 24.1 / 20.8
+// nu = 0.8:
+//   cs =  60, 5k blocks (M <=  77):     0.35 / 0.42 / 0.53 / 0.36 / 0.44
+//   cs =  80, 10k blocks (M <=  97):    0.95 / 1.06 / 1.34 / 0.93 / 1.13
+//   cs = 120, 10k blocks (M <= 137):    1.84 / 1.81 / 2.16 / 1.71 / 1.96
+//   cs = 200, 10k blocks (M <= 217):    5.37 / 4.29 / 4.60 / 4.53 / 4.84
+//   cs = 300, 20k blocks (M <= 317):    36.1 / 23.8 / 21.0 / 27.1 / 23.5
+// space-time:
+//   cs =  30, 2.5k blocks (M <=  44):   0.20 / 0.21 / 0.23 / 0.19 / 0.26
+//   cs =  47, 250 blocks (M <=  61):    .099 / .062 / .052 / .073 / .063
+//   cs =  60, 500 blocks (M <=  74):    .142 / .138 / .117 / .117 / .140
+//   cs =  60, 2.5k blocks (M <=  74):   0.51 / 0.46 / 0.47 / 0.46 / 0.59
+//   cs = 100, 2.5k blocks (M <= 114):   1.10 / 0.96 / 0.93 / 0.98 / 1.27
+//   cs = 200, 2.5k blocks (M <= 214):   5.43 / 3.23 / 3.01 / 3.91 / 4.34
+inline int lean_table(int gen, int max_m, size_t blocks)
 {
-    constexpr size_t sms = 148;
-    if (gen == kGenXYZ) return (max_m <= 90 && blocks > 2 * sms) ? 128 : 256;
-    if (max_m > 250) return (gen == kGenClosed && blocks < 16 * sms) ? 256 : 160;
-    if (max_m <= 115) return blocks > 3 * sms ? 96 : 128;
-    return (max_m <= 180 && blocks > 3 * sms && blocks <= 4 * sms) ? 160 : 128;
+    const bool few = blocks <= 2 * 148;
+    if (gen == kGenXYZ) return (max_m <= 90 && !few) ? kLean128 : kLean256;
+    if (max_m > 250) return kLean256;
+    if (few) return kLean160Wide;
+    return max_m <= 85 ? kLean96 : (max_m <= 185 ? kLean128 : kLean160);
 }
 
 // The static shared scratch the streamed path needs (a subset of
@@ -98,11 +104,6 @@ struct alignas(16) LeanShared {
     unsigned status;
     int task;
 };
-
-// Tiles of a group.  Two measured fastest (n = 1M, cs = 200: 59.1 ms at 2,
-// 63.4 at 3, 69.9 at 4 with the entries generated in shared memory: with 3 or
-// more the live fragments crowd the registers).
-constexpr int kDT = 2;
 
 __device__ __forceinline__ double2 ldcg2(const double *p)
 {
@@ -414,12 +415,8 @@ __device__ __forceinline__ void next_panel(double *nxt, const double *X, const d
 {
     const TileLane L;
     const int ntiles = (M + 8 - n0) >> 3;  // rows n0..M
-    for (int t0 = (threadIdx.x >> 5) - w0; t0 < ntiles; t0 += nw * kDT) {
-        if (t0 + nw < ntiles)
-            next_tiles<kDT, GEN>(nxt, X, Y, Z, slab, M, p, n0, t0, nw, L, mp, kw);
-        else
-            next_tiles<1, GEN>(nxt, X, Y, Z, slab, M, p, n0, t0, nw, L, mp, kw);
-    }
+    for (int t0 = (threadIdx.x >> 5) - w0; t0 < ntiles; t0 += nw)
+        next_tiles<1, GEN>(nxt, X, Y, Z, slab, M, p, n0, t0, nw, L, mp, kw);
 }
 
 // Panel p+1 (negated in nxt, rows n0..M) takes panel p's update from cur

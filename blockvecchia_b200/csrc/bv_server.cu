@@ -156,11 +156,9 @@ struct LeanServerVariant {
 };
 #define BV_LEAN_SERVER(NT, MINB) \
     {{llh_lean_server_kernel<NT, MINB, kGenClosed>, llh_lean_server_kernel<NT, MINB, kGenGeneral>}, NT}
-static const LeanServerVariant kLeanServer[] = {
-    BV_LEAN_SERVER(96, 4),
-    BV_LEAN_SERVER(128, 3),
+static const LeanServerVariant kLeanServer[kLeanShapes] = {  // in the order of LeanShape
+    BV_LEAN_SERVER(96, 5), BV_LEAN_SERVER(160, 3), BV_LEAN_SERVER(256, 2), BV_LEAN_SERVER(128, 4),
     BV_LEAN_SERVER(160, 2),
-    BV_LEAN_SERVER(256, 2),
 };
 
 }  // namespace bv
@@ -405,8 +403,7 @@ struct LeanLaunch {
 
 bool lean_launch_for(const bv_server *S, int gen, int max_m, size_t blocks, LeanLaunch &ll)
 {
-    const int t = lean_table_threads(gen, max_m, blocks);
-    ll.v = &kLeanServer[t == 96 ? 0 : (t == 128 ? 1 : (t == 160 ? 2 : 3))];
+    ll.v = &kLeanServer[lean_table(gen, max_m, blocks)];
     ll.smem = std::max<size_t>(lean_smem(gen, max_m, 0, S->lean_avail), kReduceScratchBytes);
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ll.v->kernel[gen], ll.v->threads, ll.smem) != cudaSuccess ||
@@ -820,7 +817,7 @@ extern "C" int bv_server_create(const bv_server_opts *opts, bv_server **out)
     // The streamed kernel: the handles' limit, and its shared memory allowed.
     {
         cudaFuncAttributes fl;
-        BV_CUDA_TRY(cudaFuncGetAttributes(&fl, kLeanServer[3].kernel[kGenClosed]));
+        BV_CUDA_TRY(cudaFuncGetAttributes(&fl, kLeanServer[kLean256].kernel[kGenClosed]));
         const size_t avail = (size_t)optin - fl.sharedSizeBytes;
         S->lean_avail = avail;
         S->lean_limit = big_max_m_for_bytes(avail, 0, 0, 0);
@@ -846,7 +843,7 @@ extern "C" int bv_server_create(const bv_server_opts *opts, bv_server **out)
         // blocks of 50) at every table point, so that batches of such jobs
         // allocate nothing; larger batches grow them.
         size_t pre = 0;
-        for (int m : {115, 250, std::min(350, S->lean_limit)}) {
+        for (int m : {85, 185, 250, std::min(350, S->lean_limit)}) {
             size_t both = 0;
             for (int g = 0; g < 2; ++g) {
                 LeanLaunch ll;

@@ -171,11 +171,10 @@ typedef struct {
     int streamed_threads; /* threads per CTA of that kernel (0: none)       */
     int streamed_variant; /* its variant, an index into tune_ms             */
     double tune_ms[6];   /* with bv_opts.tune: the streamed kernel's time on
-                            the first evaluation per variant: 96 threads x 4
-                            CTAs per SM, 160 x 3, 256 x 2, 128 x 3, 160 x 2
-                            and 256 x 1 (with a third coordinate 96 x 5 and
-                            128 x 4; blocks up to M = 48 at a closed-form nu
-                            one per warp in the last's place; 0 where not
+                            the first evaluation per variant: 96 threads x 5
+                            CTAs per SM, 160 x 3, 256 x 2, 128 x 4, 160 x 2
+                            and 256 x 1 (blocks up to M = 48 at a closed-form
+                            nu one per warp in the last's place; 0 where not
                             timed)                                           */
 } bv_status;
 
