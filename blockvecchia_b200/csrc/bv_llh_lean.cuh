@@ -61,21 +61,21 @@ enum LeanShape : int { kLean96 = 0, kLean160 = 1, kLean256 = 2, kLean128 = 3, kL
 // blocks per SM wants each block short.  Entries generated through shared
 // memory (a third coordinate) are a larger share of the update warps' work.
 // Kernel ms at 96 x 5 / 160 x 3 / 256 x 2 / 128 x 4 / 160 x 2:
-//   cs =  60, 150 blocks (M <=  82):    .041 / .035 / .033 / .037 / .032
+//   cs =  60, 150 blocks (M <=  82):    .041 / .036 / .034 / .036 / .031
 //   cs = 120, 300 blocks (M <= 137):    .086 / .064 / .064 / .070 / .061
 //   cs = 120, 500 blocks (M <= 137):    .099 / .107 / .109 / .092 / .107
-//   cs =  60, 5k blocks (M <=  77):     0.25 / 0.31 / 0.42 / 0.27 / 0.38
+//   cs =  60, 5k blocks (M <=  77):     0.24 / 0.32 / 0.42 / 0.26 / 0.37
 //   cs =  80, 10k blocks (M <=  97):    0.74 / 0.81 / 1.08 / 0.73 / 1.01
-//   cs = 120, 20k blocks (M <= 137):    2.91 / 2.83 / 3.37 / 2.67 / 3.34
+//   cs = 120, 20k blocks (M <= 137):    2.54 / 2.73 / 3.41 / 2.45 / 3.31
 //   cs = 160, 10k blocks (M <= 177):    2.59 / 2.33 / 2.58 / 2.22 / 2.76
-//   cs = 200, 100k blocks (M <= 217):   47.5 / 34.7 / 37.4 / 37.8 / 42.9
+//   cs = 200, 100k blocks (M <= 217):   47.8 / 34.6 / 37.2 / 38.1 / 42.9
 //   cs = 240, 10k blocks (M <= 257):    7.28 / 5.21 / 5.26 / 5.77 / 6.25
 //   cs = 300, 1.5k blocks (M <= 322):   2.91 / 1.87 / 1.45 / 2.09 / 1.86
 //   cs = 300, 20k blocks (M <= 317):    33.4 / 20.9 / 17.1 / 24.1 / 20.8
 // nu = 0.8:
 //   cs =  60, 5k blocks (M <=  77):     0.35 / 0.42 / 0.53 / 0.36 / 0.44
 //   cs =  80, 10k blocks (M <=  97):    0.95 / 1.06 / 1.34 / 0.93 / 1.13
-//   cs = 120, 10k blocks (M <= 137):    1.84 / 1.81 / 2.16 / 1.71 / 1.96
+//   cs = 120, 10k blocks (M <= 137):    1.76 / 1.70 / 2.05 / 1.59 / 1.96
 //   cs = 200, 10k blocks (M <= 217):    5.37 / 4.29 / 4.60 / 4.53 / 4.84
 //   cs = 300, 20k blocks (M <= 317):    36.1 / 23.8 / 21.0 / 27.1 / 23.5
 // space-time:
@@ -476,91 +476,97 @@ __device__ __forceinline__ void store_row(double *row, int r, const double (&v)[
 }
 
 // The diagonal block of panel p (rows k0.., kb <= 16 columns) and the 16 rows
-// below it, by one warp: lane r holds row k0 + r in v (zeros above the
-// diagonal and beyond the block).  The element operations and their order are
-// factor_rows' (lagged Crout: the products over k < c - 1 in four partial
-// sums by k mod 4, the k = c - 1 product last).
+// below it, by one warp, in place: lane r owns row k0 + r of cur.  The element
+// operations and their order are factor_rows' (lagged Crout: the products over
+// k < c - 1 in four partial sums by k mod 4, the k = c - 1 product last).
 //
 // The warp's time is the dependent chain of 16 pivots (an FP64 rsqrt is ~60
-// cycles, a shuffle 26 and more when the SM's shared-memory pipe is busy), so
-// four columns are done per round: the lanes' partial sums over the earlier
-// columns are formed by themselves, the 4 x 4 diagonal block's go to every
-// lane through `ex`, and every lane factors that block redundantly and
-// applies it to its own row -- two shared-memory exchanges per four pivots
-// instead of eight to thirty-two shuffles per pivot, no divergent branches.
-// Alone on an SM sub-partition: 4.6k cycles per panel with shuffles and a
-// guard per pivot, 3.5k this way, and fewer shared-memory operations for the
-// other CTAs' warps to queue behind.
+// cycles, a shuffle 26 and more when the SM's shared-memory pipe is busy) and
+// the fetch of its code.  Four columns are done per round, one round's code
+// looped: the lanes' partial sums over the earlier columns are formed by
+// themselves, the 4 x 4 diagonal block's go to every lane through `ex`, and
+// every lane factors that block redundantly and applies it to its own row --
+// two shared-memory exchanges per four pivots instead of eight to thirty-two
+// shuffles per pivot, no divergent branches, and the finished columns read
+// back from the panel instead of held in registers (a lane above its diagonal
+// reads what it finds there: its entry is set to zero).
 //
-// Lt receives the factor transposed (zeros above the diagonal and in columns
-// beyond kb); myinv is 1 / L_rr of a lane's own pivot (0: failed).
-__device__ __forceinline__ unsigned factor_panel(int k0, int kb, int mc, double (&v)[kNB], double &myinv,
-                                                 double (*Lt)[kNB], double (*ex)[8])
+// sh.Lt receives the factor transposed (zeros above the diagonal and beyond
+// kb), sh.inv 1 / L_qq (0: failed).
+//
+// kUnroll: 1, one round's code (n = 200k, cs = 120, 128 x 4: 2.67 ms with an
+// unrolled column-by-column factorization by shuffles, 2.45 with this), or 4,
+// unrolled for the shapes that leave few warps on an SM (150 blocks, cs = 60,
+// 160 x 2: .0356 looped, .0312 unrolled).
+template <int kUnroll>
+static __device__ __forceinline__ unsigned factor_phase(double *cur, int M, int k0, int kb, int mc,
+                                                        LeanShared &sh)
 {
     const int lane = threadIdx.x & 31;
     const bool low = lane < kNB;
+    const bool valid = low ? lane < kb : (kb == kNB && k0 + lane <= M);
+    const int x = (lane & 3) << 2;  // k0 is a multiple of 16
+    double *row = cur + (valid ? lane : 0) * 16;
     unsigned st = 0;
-    myinv = 0.0;
-#pragma unroll
+#pragma unroll kUnroll
     for (int c0 = 0; c0 < kNB; c0 += 4) {
-        // Columns c0, c0+1: complete sums but for the products of this round;
-        // c0+2, c0+3: partial sums 0, 1 and the sum of 2 and 3.
-        double s0, s1, g2[3], g3[3];
-        if (c0 == 0) {
-            s0 = v[0];
-            s1 = v[1];
-            g2[0] = v[2];
-            g3[0] = v[3];
-            g2[1] = g2[2] = g3[1] = g3[2] = 0.0;
-        } else {
-            double a[4][4], last = 0.0;
+        double a[4][4], last = 0.0, vlast = 0.0;
+        {
+            const double2 u0 = ld2(row + (c0 ^ x)), u1 = ld2(row + ((c0 ^ x) + 2));
+            const double u[4] = {u0.x, u0.y, u1.x, u1.y};
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                a[c][0] = v[c0 + c];
+                a[c][0] = (valid && c0 + c < kb && (!low || c0 + c <= lane)) ? u[c] : 0.0;
                 a[c][1] = a[c][2] = a[c][3] = 0.0;
             }
-#pragma unroll
-            for (int k = 0; k < c0; ++k) {
-                // Four columns' loads at a time (more would spill).
-                if ((k & 3) == 0) asm volatile("" ::: "memory");
-                const double2 x = ld2(&Lt[k][c0]), y = ld2(&Lt[k][c0 + 2]);
-                if (k == c0 - 1)
-                    last = x.x;
-                else
-                    a[0][k & 3] = fma(-v[k], x.x, a[0][k & 3]);
-                a[1][k & 3] = fma(-v[k], x.y, a[1][k & 3]);
-                a[2][k & 3] = fma(-v[k], y.x, a[2][k & 3]);
-                a[3][k & 3] = fma(-v[k], y.y, a[3][k & 3]);
-            }
-            s0 = fma(-v[c0 - 1], last, (a[0][0] + a[0][1]) + (a[0][2] + a[0][3]));
-            s1 = (a[1][0] + a[1][1]) + (a[1][2] + a[1][3]);
-            g2[0] = a[2][0];
-            g2[1] = a[2][1];
-            g2[2] = a[2][2] + a[2][3];
-            g3[0] = a[3][0];
-            g3[1] = a[3][1];
-            g3[2] = a[3][2] + a[3][3];
         }
+#pragma unroll kUnroll
+        for (int k = 0; k < c0; k += 4) {
+            const bool end = k + 4 == c0;
+            const double2 v0 = ld2(row + (k ^ x)), v1 = ld2(row + ((k ^ x) + 2));
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const double v = (j & 2) ? ((j & 1) ? v1.y : v1.x) : ((j & 1) ? v0.y : v0.x);
+                const double2 p = ld2(&sh.Lt[k + j][c0]), q = ld2(&sh.Lt[k + j][c0 + 2]);
+                if (j == 3 && end) {  // column c0's last product follows its sum
+                    last = p.x;
+                    vlast = v;
+                } else {
+                    a[0][j] = fma(-v, p.x, a[0][j]);
+                }
+                a[1][j] = fma(-v, p.y, a[1][j]);
+                a[2][j] = fma(-v, q.x, a[2][j]);
+                a[3][j] = fma(-v, q.y, a[3][j]);
+            }
+        }
+        // Columns c0, c0+1: complete sums but for the products of this round;
+        // c0+2, c0+3: partial sums 0, 1 and the sum of 2 and 3.
+        const double s0 = fma(-vlast, last, (a[0][0] + a[0][1]) + (a[0][2] + a[0][3]));
+        const double s1 = (a[1][0] + a[1][1]) + (a[1][2] + a[1][3]);
+        const double g2[3] = {a[2][0], a[2][1], a[2][2] + a[2][3]};
+        const double g3[3] = {a[3][0], a[3][1], a[3][2] + a[3][3]};
         if (lane >= c0 && lane < c0 + 4) {
-            double2 *e = reinterpret_cast<double2 *>(ex[lane - c0]);
+            double2 *e = reinterpret_cast<double2 *>(sh.ex[lane - c0]);
             e[0] = make_double2(s0, s1);
             e[1] = make_double2(g2[0], g2[1]);
             e[2] = make_double2(g2[2], g3[0]);
             e[3] = make_double2(g3[1], g3[2]);
         }
         __syncwarp();
-        // Read in two parts: all at once would spill at 128 registers.
-        const double e0 = ex[0][0];
-        const double2 e1 = ld2(&ex[1][0]), e2a = ld2(&ex[2][0]), e3a = ld2(&ex[3][0]);
+        const double2 e1 = ld2(&sh.ex[1][0]);
+        const double2 e2a = ld2(&sh.ex[2][0]), e2b = ld2(&sh.ex[2][2]);
+        const double2 e3a = ld2(&sh.ex[3][0]), e3b = ld2(&sh.ex[3][2]), e3c = ld2(&sh.ex[3][4]),
+                      e3d = ld2(&sh.ex[3][6]);
+        const double e0 = sh.ex[0][0], e2c = sh.ex[2][4];
         double piv[4], inv[4], w[4];
         bool ok[4];
         // A failed pivot's column is zero below it; rsqrt of 1 keeps the
         // evaluation branch-free.
-        auto pivot = [&](int c, double x) {
-            piv[c] = x;
-            ok[c] = x > 0.0;
-            const double y = rsqrt(ok[c] ? x : 1.0);
-            inv[c] = ok[c] ? y : 0.0;
+        auto pivot = [&](int c, double y) {
+            piv[c] = y;
+            ok[c] = y > 0.0;
+            const double z = rsqrt(ok[c] ? y : 1.0);
+            inv[c] = ok[c] ? z : 0.0;
         };
         pivot(0, e0);
         const double l10 = e1.x * inv[0], l20 = e2a.x * inv[0], l30 = e3a.x * inv[0];
@@ -568,9 +574,6 @@ __device__ __forceinline__ unsigned factor_panel(int k0, int kb, int mc, double 
         pivot(1, fma(-l10, l10, e1.y));
         const double l21 = fma(-l20, l10, e2a.y) * inv[1], l31 = fma(-l30, l10, e3a.y) * inv[1];
         w[1] = fma(-w[0], l10, s1) * inv[1];
-        asm volatile("" ::: "memory");
-        const double2 e2b = ld2(&ex[2][2]), e3b = ld2(&ex[3][2]), e3c = ld2(&ex[3][4]), e3d = ld2(&ex[3][6]);
-        const double e2c = ex[2][4];
         pivot(2, fma(-l21, l21, (fma(-l20, l20, e2b.x) + e2b.y) + e2c));
         const double l32 = fma(-l31, l21, (fma(-l30, l20, e3b.x) + e3b.y) + e3c.x) * inv[2];
         w[2] = fma(-w[1], l21, (fma(-w[0], l20, g2[0]) + g2[1]) + g2[2]) * inv[2];
@@ -580,80 +583,16 @@ __device__ __forceinline__ unsigned factor_panel(int k0, int kb, int mc, double 
         for (int c = 0; c < 4; ++c) {
             const int q = c0 + c;
             if (!ok[c] && q < kb) st |= (k0 + q < mc) ? 1u : 2u;
-            const double dq = ok[c] ? piv[c] * inv[c] : piv[c];
-            v[q] = (lane > q) ? w[c] : ((lane == q) ? dq : v[q]);
-            if (lane == q) myinv = inv[c];
-            if (low) Lt[q][lane] = (lane < kb) ? v[q] : 0.0;
+            w[c] = (lane > q) ? w[c] : ((lane == q) ? (ok[c] ? piv[c] * inv[c] : piv[c]) : 0.0);
+            if (low) sh.Lt[q][lane] = (valid && q < kb) ? w[c] : 0.0;
+            if (lane == q) sh.inv[q] = (q < kb) ? inv[c] : 0.0;
+        }
+        if (valid && lane >= c0) {
+            *reinterpret_cast<double2 *>(row + (c0 ^ x)) = make_double2(w[0], w[1]);
+            *reinterpret_cast<double2 *>(row + ((c0 ^ x) + 2)) = make_double2(w[2], w[3]);
         }
         __syncwarp();
     }
-    return st;
-}
-
-// The same with one column at a time and shuffles, in half the registers (62
-// against 110: no spills in kernels limited to 128; 3.6k cycles per panel
-// alone, more than factor_panel's when the shared-memory pipe is loaded).
-__device__ __forceinline__ unsigned factor_panel_narrow(int k0, int kb, int mc, double (&v)[kNB],
-                                                        double &myinv, double (*Lt)[kNB])
-{
-    const int lane = threadIdx.x & 31;
-    const bool low = lane < kNB;
-    unsigned st = 0;
-    myinv = 0.0;
-    double pre = v[0];
-#pragma unroll
-    for (int q = 0; q < kNB; ++q) {
-        const double preq = __shfl_sync(0xffffffffu, pre, q);
-        double s = pre, piv = preq;
-        if (q > 0) {
-            const double l = __shfl_sync(0xffffffffu, v[q - 1], q);
-            s = fma(-v[q - 1], l, s);
-            piv = fma(-l, l, preq);
-        }
-        const bool ok = piv > 0.0;
-        double inv = rsqrt(ok ? piv : 1.0);
-        inv = ok ? inv : 0.0;
-        if (q + 1 < kNB) {
-            double s4[4] = {v[q + 1], 0.0, 0.0, 0.0};
-#pragma unroll
-            for (int k = 0; k < q; ++k) {
-                const double lk = __shfl_sync(0xffffffffu, v[k], q + 1);
-                s4[k & 3] = fma(-v[k], lk, s4[k & 3]);
-            }
-            pre = (s4[0] + s4[1]) + (s4[2] + s4[3]);
-        }
-        if (!ok && q < kb) st |= (k0 + q < mc) ? 1u : 2u;
-        const double dq = ok ? piv * inv : piv;
-        v[q] = (lane > q) ? s * inv : ((lane == q) ? dq : v[q]);
-        if (lane == q) myinv = inv;
-        if (low) Lt[q][lane] = (lane < kb) ? v[q] : 0.0;
-    }
-    return st;
-}
-
-// The factor warp's part of panel p (rows k0.. in cur): lane r < kb owns row
-// k0+r of the diagonal block; with a full panel the upper lanes solve the
-// next 16 rows on the same chain, so the substitution starts 16 rows on.
-template <bool kNarrow>
-__device__ __forceinline__ unsigned factor_phase(double *cur, int M, int k0, int kb, int mc, LeanShared &sh)
-{
-    const int lane = threadIdx.x & 31;
-    const bool low = lane < kNB;
-    const int row = k0 + lane;
-    const bool valid = low ? lane < kb : (kb == kNB && row <= M);
-    double *rowp = cur + (valid ? lane : 0) * 16;
-    double v[kNB], myinv;
-    load_row(rowp, valid ? row : k0, v);
-#pragma unroll
-    for (int c = 0; c < kNB; ++c)
-        if (!(valid && c < kb && (!low || c <= lane))) v[c] = 0.0;
-    unsigned st;
-    if constexpr (kNarrow)
-        st = factor_panel_narrow(k0, kb, mc, v, myinv, sh.Lt);
-    else
-        st = factor_panel(k0, kb, mc, v, myinv, sh.Lt, sh.ex);
-    if (valid) store_row(rowp, row, v);
-    if (low) sh.inv[lane] = (lane < kb) ? myinv : 0.0;
     return st;
 }
 
@@ -823,7 +762,7 @@ __device__ __forceinline__ void process_block_lean(const LlhArgs &a, const Mater
         const int kb1 = max(0, min(kNB, M - n0));  // its width
         if (warp == 0) {
             if (!kFirst || p >= 0)
-                st |= factor_phase<(NT * MINB > 384)>(cur, M, k0, kb, mc, sh);
+                st |= factor_phase<(NT * MINB > 320) ? 1 : 4>(cur, M, k0, kb, mc, sh);
         } else if (kb1 > 0) {
             if constexpr (kXYZ3) {
                 const int u = tid - 32;
@@ -979,7 +918,7 @@ __device__ __forceinline__ void process_block_warp(const LlhArgs &a, const Mater
         const int k0 = max(0, p * kNB), kb = (p < 0) ? 0 : min(kNB, M - k0), n0 = k0 + kb;
         if (p >= 0) {
             double *cur = slab + big_panel_base(p, Mp);
-            st |= factor_phase<false>(cur, M, k0, kb, mc, sh);
+            st |= factor_phase<4>(cur, M, k0, kb, mc, sh);
             __syncwarp();
             for (int r = k0 + (kb == kNB ? 2 * kNB : kb) + lane; r < Mp; r += 32)
                 solve_row(sh, cur + (r - k0) * 16, r);
