@@ -157,12 +157,26 @@ void set_error(const char *fmt, ...)
 }
 const char *get_error() { return g_err; }
 
+// Start of an evaluation: the parameters from pinned host memory and zeroed
+// work counters, in one launch (a copy and a memset node, and a copy node for
+// the result, cost a 2k-point evaluation 10 of its 74 us).
+constexpr int kBeginThreads = 64;
+static_assert(sizeof(MaternParams) % 4 == 0 && sizeof(MaternParams) / 4 <= kBeginThreads, "one word per thread");
+__global__ void __launch_bounds__(kBeginThreads) eval_begin_kernel(const MaternParams *src, MaternParams *dst,
+                                                                  unsigned *counters, int n)
+{
+    const int t = threadIdx.x;
+    if (t < (int)(sizeof(MaternParams) / 4))
+        reinterpret_cast<unsigned *>(dst)[t] = reinterpret_cast<const volatile unsigned *>(src)[t];
+    for (int i = t; i < n; i += kBeginThreads) counters[i] = 0u;
+}
+
 __global__ void __launch_bounds__(kReduceThreads) reduce_kernel(const double *v,
                                                                 const unsigned *st, int n,
                                                                 EvalResult *out)
 {
     __shared__ __align__(16) unsigned char scratch[kReduceScratchBytes];
-    reduce_blocks(v, st, n, out, scratch);
+    reduce_blocks<true>(v, st, n, out, scratch);
 }
 
 }  // namespace bv
@@ -198,7 +212,6 @@ struct bv_handle {
     double tune_ms[kNumLean] = {};
     MaternParams *d_mp = nullptr;
     double2 *d_ktab = nullptr;  // the general-nu table (bv_ktab.cuh)
-    EvalResult *d_res = nullptr;
     MixedWork mixed;  // mixed-precision scratch (bv_llh_mixed.cuh)
     // pinned host
     MaternParams *h_mp = nullptr;
@@ -232,6 +245,7 @@ struct bv_handle {
     cudaStream_t own_stream = nullptr;  // the handle's stream; `stream` may be a caller's
     // status
     bv_status status{};
+    bool timed = false;  // status.device_ms / kernel_ms are to be read from the events
     int iterations = 0;
 };
 
@@ -264,7 +278,6 @@ static void handle_free(bv_handle *h)
     cudaFree(h->d_slab_lean);
     cudaFree(h->d_mp);
     cudaFree(h->d_ktab);
-    cudaFree(h->d_res);
     mixed_free(h->mixed);
     cudaFreeHost(h->h_mp);
     cudaFreeHost(h->h_res);
@@ -634,8 +647,8 @@ static int eval_kind(const bv_handle *h)
 // One evaluation on stream s; kind: 0 a closed-form nu, 1 a general nu.
 static int enqueue_eval(bv_handle *h, cudaStream_t s, int kind)
 {
-    BV_CUDA_TRY(cudaMemcpyAsync(h->d_mp, h->h_mp, sizeof(MaternParams), cudaMemcpyHostToDevice, s));
-    BV_CUDA_TRY(cudaMemsetAsync(h->d_counters, 0, sizeof(unsigned) * std::max<size_t>(1, h->launches.size()), s));
+    eval_begin_kernel<<<1, kBeginThreads, 0, s>>>(h->h_mp, h->d_mp, h->d_counters, (int)h->launches.size());
+    BV_CUDA_TRY(cudaGetLastError());
     BV_CUDA_TRY(record_timing(h->evk0, s));
     if (kind == 1) {
         ktab_kernel<<<kTabCtas, kTabThreads, 0, s>>>(h->d_mp, h->d_ktab);
@@ -715,9 +728,9 @@ static int enqueue_eval(bv_handle *h, cudaStream_t s, int kind)
         }
     }
     BV_CUDA_TRY(record_timing(h->evk1, s));
-    reduce_kernel<<<1, kReduceThreads, 0, s>>>(h->d_block_llk, h->d_block_status, h->bc, h->d_res);
+    // The result record goes straight to the pinned host copy.
+    reduce_kernel<<<1, kReduceThreads, 0, s>>>(h->d_block_llk, h->d_block_status, h->bc, h->h_res);
     BV_CUDA_TRY(cudaGetLastError());
-    BV_CUDA_TRY(cudaMemcpyAsync(h->h_res, h->d_res, sizeof(EvalResult), cudaMemcpyDeviceToHost, s));
     return BV_OK;
 }
 
@@ -842,7 +855,6 @@ extern "C" int bv_create(const bv_layout *L, const bv_opts *opts, bv_handle **ou
     BV_CUDA_H(cudaMalloc(&h->d_block_status, bc * sizeof(unsigned)));
     BV_CUDA_H(cudaMalloc(&h->d_mp, sizeof(MaternParams)));
     BV_CUDA_H(cudaMalloc(&h->d_ktab, kTabEntries * sizeof(double2)));
-    BV_CUDA_H(cudaMalloc(&h->d_res, sizeof(EvalResult)));
     BV_CUDA_H(cudaMallocHost(&h->h_mp, sizeof(MaternParams)));
     BV_CUDA_H(cudaMallocHost(&h->h_res, sizeof(EvalResult)));
     BV_CUDA_H(cudaMemcpy(h->d_x, L->x, n * sizeof(double), cudaMemcpyHostToDevice));
@@ -1044,9 +1056,7 @@ static int eval_locked(bv_handle *h, const double *theta, double *llk)
     }
     BV_CUDA_TRY(cudaEventRecord(h->ev1, h->stream));
     BV_CUDA_TRY(cudaStreamSynchronize(h->stream));
-    float ms = 0.f, kms = 0.f;
-    cudaEventElapsedTime(&ms, h->ev0, h->ev1);
-    cudaEventElapsedTime(&kms, h->evk0, h->evk1);
+    h->timed = true;
     const EvalResult r = *h->h_res;
     bv_status &s = h->status;
     s.blocks = h->owned;
@@ -1075,8 +1085,6 @@ static int eval_locked(bv_handle *h, const double *theta, double *llk)
     s.streamed_variant = lk ? lk->variant : -1;
     for (int i = 0; i < kNumLean; ++i) s.tune_ms[i] = h->tune_ms[i];
     s.llk = r.llk;
-    s.device_ms = ms;
-    s.kernel_ms = kms;
     double v = r.llk;
     const bool failed = (r.cond_fail + r.schur_fail + r.nonfinite) > 0 || !std::isfinite(v);
     if (failed && h->opts.on_failure == BV_FAIL_NEGINF) v = -HUGE_VAL;
@@ -1179,6 +1187,14 @@ extern "C" int bv_get_status(bv_handle *h, bv_status *st)
 {
     if (!h || !st) return BV_E_INVALID;
     std::lock_guard<std::mutex> lk(h->mu);
+    if (h->timed) {  // the last evaluation's events have completed
+        float ms = 0.f, kms = 0.f;
+        cudaEventElapsedTime(&ms, h->ev0, h->ev1);
+        cudaEventElapsedTime(&kms, h->evk0, h->evk1);
+        h->status.device_ms = ms;
+        h->status.kernel_ms = kms;
+        h->timed = false;
+    }
     *st = h->status;
     return BV_OK;
 }

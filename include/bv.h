@@ -164,7 +164,8 @@ typedef struct {
     int failed;          /* blocks with a failed pivot in either factor
                             (cond_fail and schur_fail may count one block
                             twice; this counts it once)                      */
-    int launches;        /* kernel launches per evaluation                   */
+    int launches;        /* kernel launches per evaluation, the parameters'
+                            set-up (and a general nu's table) not counted    */
     int streamed_blocks; /* FP64 path: blocks on the multi-CTA streamed
                             kernel (the rest on the persistent kernel);
                             0 for the mixed path                             */
