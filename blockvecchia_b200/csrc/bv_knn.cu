@@ -135,11 +135,19 @@ __global__ void __launch_bounds__(kBoxThreads) knn_box_kernel(const double *x, c
 // ... and the grid's shape: square cells, at most ncell of them.
 __global__ void knn_grid_kernel(const double *part, int ncell, KnnGrid *grid)
 {
-    if (threadIdx.x != 0) return;
-    double b[4] = {part[0], part[1], part[2], part[3]};
-    for (int c = 1; c < kBoxCtas; ++c)
+    double b[4] = {INFINITY, -INFINITY, INFINITY, -INFINITY};
+    for (int c = threadIdx.x; c < kBoxCtas; c += 32)
+#pragma unroll
         for (int k = 0; k < 4; ++k)
             b[k] = (k & 1) ? fmax(b[k], part[4 * c + k]) : fmin(b[k], part[4 * c + k]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const double v = __shfl_xor_sync(0xffffffffu, b[k], o);
+            b[k] = (k & 1) ? fmax(b[k], v) : fmin(b[k], v);
+        }
+    if (threadIdx.x != 0) return;
     KnnGrid g;
     g.x0 = b[0];
     g.y0 = b[2];
@@ -185,16 +193,17 @@ __global__ void knn_cells_kernel(const double *x, const double *y, const double 
 
 // Exclusive prefix sums of the counts by one CTA: start[0 .. ncell] and a copy
 // in the counts' place (the scatter's cursors).
+constexpr int kScanItems = 16;  // cells of a thread at a time
 __global__ void __launch_bounds__(1024) knn_scan_kernel(int *count, int *start, int ncell)
 {
     __shared__ int warp_sum[32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int carry = 0;
-    for (int base = 0; base < ncell; base += 4096) {
-        int v[4], t = 0;
+    for (int base = 0; base < ncell; base += 1024 * kScanItems) {
+        int v[kScanItems], t = 0;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int i = base + tid * 4 + u;
+        for (int u = 0; u < kScanItems; ++u) {
+            const int i = base + tid * kScanItems + u;
             v[u] = (i < ncell) ? count[i] : 0;
             t += v[u];
         }
@@ -213,8 +222,8 @@ __global__ void __launch_bounds__(1024) knn_scan_kernel(int *count, int *start, 
         }
         int run = before + incl - t;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int i = base + tid * 4 + u;
+        for (int u = 0; u < kScanItems; ++u) {
+            const int i = base + tid * kScanItems + u;
             if (i < ncell) {
                 start[i] = run;
                 count[i] = run;
@@ -819,28 +828,43 @@ int knn_device(const double *d_x, const double *d_y, const double *d_z, int n, i
         rc = BV_E_CUDA;
     };
     cudaError_t e;
-    if ((e = cudaMalloc(&d_c, sizeof(double) * 3 * (size_t)bc)) != cudaSuccess) {
-        fail(e, "cudaMalloc");
-        return rc;
-    }
     // Blocks 1..bc-1 to select for, largest prefix first (all, or the mask's).
     std::vector<int> list;
     if (mask) {
         for (int b = bc - 1; b >= 1; --b)
             if (mask[b]) list.push_back(b);
     }
-    // counter, error, heavy_count, the heavy list (bc entries), the block list
-    if ((e = cudaMalloc(&d_counter, sizeof(unsigned) * 3 + sizeof(int) * (size_t)bc * 2)) != cudaSuccess) {
-        cudaFree(d_c);
+    // One scratch allocation (an allocation and its release cost ~0.2 ms, as
+    // much as a small selection): the centroids; with a grid the locations in
+    // cell order, partial boxes and the grid; then ints: counter, error,
+    // heavy_count, the heavy list (bc entries), the block list, and the grid's
+    // cell starts, counts and indices.
+    bool use_grid = geo != kGeoEarth && n >= kGridMinN;
+    const int ncell = n / kGridOcc;
+    const size_t nc = 3 * (size_t)bc;
+    size_t ngd = (size_t)n * (d_z ? 3 : 2) + 4 * kBoxCtas + sizeof(KnnGrid) / sizeof(double) + 1;
+    size_t ngi = (size_t)n + 2 * (size_t)ncell + 1;
+    auto scratch = [&] {
+        if (!use_grid) ngd = ngi = 0;
+        return cudaMalloc(&d_c, (nc + ngd) * sizeof(double) + (3 + 2 * (size_t)bc + ngi) * sizeof(int));
+    };
+    e = scratch();
+    if (e == cudaErrorMemoryAllocation && use_grid) {  // no room for the grid: scan the prefixes
+        cudaGetLastError();
+        use_grid = false;
+        e = scratch();
+    }
+    if (e != cudaSuccess) {
         fail(e, "cudaMalloc");
         return rc;
     }
+    double *const d_grid = d_c + nc;
+    d_counter = reinterpret_cast<unsigned *>(d_grid + ngd);
     d_err = reinterpret_cast<int *>(d_counter + 1);
     unsigned *d_heavy_count = d_counter + 2;
     int *d_heavy = reinterpret_cast<int *>(d_counter + 3);
     int *d_list = d_heavy + bc;
     KnnHeavyScratch sc{nullptr, nullptr, nullptr};
-    double *d_grid = nullptr;
     do {
         if ((e = cudaMemcpyAsync(d_c, cx, sizeof(double) * bc, cudaMemcpyHostToDevice, s)) ||
             (e = cudaMemcpyAsync(d_c + bc, cy, sizeof(double) * bc, cudaMemcpyHostToDevice, s)) ||
@@ -872,20 +896,11 @@ int knn_device(const double *d_x, const double *d_y, const double *d_z, int n, i
         ka.nlist = (int)list.size();
         ka.grid = nullptr;
         ka.n = n;
-        if (geo != kGeoEarth && n >= kGridMinN) {
-            // One scratch allocation: the locations in cell order, partial
-            // boxes, the grid, cell starts and counts, indices.
-            const int ncell = n / kGridOcc;
-            const size_t nd = (size_t)n * (d_z ? 3 : 2) + 4 * kBoxCtas + sizeof(KnnGrid) / sizeof(double) + 1;
-            const size_t ni = (size_t)n + 2 * (size_t)ncell + 1;
-            if ((e = cudaMalloc(&d_grid, nd * sizeof(double) + ni * sizeof(int)))) {
-                fail(e, "cudaMalloc (grid)");
-                break;
-            }
+        if (use_grid) {
             double *sx = d_grid, *sy = sx + n, *sz = sy + n;
             double *part = d_z ? sz + n : sz;
             KnnGrid *grid = reinterpret_cast<KnnGrid *>(part + 4 * kBoxCtas);
-            int *start = reinterpret_cast<int *>(d_grid + nd);
+            int *start = d_list + bc;
             int *cells = start + ncell + 1, *sidx = cells + ncell;
             if ((e = cudaMemsetAsync(cells, 0, sizeof(int) * (size_t)ncell, s))) {
                 fail(e, "memset");
@@ -960,8 +975,6 @@ int knn_device(const double *d_x, const double *d_y, const double *d_z, int n, i
         }
     } while (0);
     cudaFree(d_c);
-    cudaFree(d_counter);
-    cudaFree(d_grid);
     cudaFree(sc.key);
     cudaFree(sc.idx);
     cudaFree(sc.pos);
@@ -1014,14 +1027,16 @@ static int knn_host(const double *x, const double *y, const double *z, int n, in
     int rc = BV_OK;
     cudaError_t e;
     do {
-        if ((e = cudaMalloc(&d_x, sizeof(double) * n)) || (e = cudaMalloc(&d_y, sizeof(double) * n)) ||
-            (z && (e = cudaMalloc(&d_z, sizeof(double) * n))) ||
-            (e = cudaMalloc(&d_acc, sizeof(int) * (bc + 1))) ||
-            (e = cudaMalloc(&d_knn, sizeof(int) * (size_t)bc * cs))) {
+        const size_t nd = (size_t)n * (z ? 3 : 2);
+        if ((e = cudaMalloc(&d_x, nd * sizeof(double) + ((size_t)bc + 1 + (size_t)bc * cs) * sizeof(int)))) {
             set_error("bv_knn: cudaMalloc: %s", cudaGetErrorString(e));
             rc = (e == cudaErrorMemoryAllocation) ? BV_E_NOMEM : BV_E_CUDA;
             break;
         }
+        d_y = d_x + n;
+        d_z = z ? d_y + n : nullptr;
+        d_acc = reinterpret_cast<int *>(d_x + nd);
+        d_knn = d_acc + bc + 1;
         if ((e = cudaMemcpyAsync(d_x, x, sizeof(double) * n, cudaMemcpyHostToDevice, s)) ||
             (e = cudaMemcpyAsync(d_y, y, sizeof(double) * n, cudaMemcpyHostToDevice, s)) ||
             (z && (e = cudaMemcpyAsync(d_z, z, sizeof(double) * n, cudaMemcpyHostToDevice, s))) ||
@@ -1056,10 +1071,6 @@ static int knn_host(const double *x, const double *y, const double *z, int n, in
         }
     } while (0);
     cudaFree(d_x);
-    cudaFree(d_y);
-    cudaFree(d_z);
-    cudaFree(d_acc);
-    cudaFree(d_knn);
     cudaStreamDestroy(s);
     return rc;
 }
