@@ -66,18 +66,18 @@ enum LeanShape : int { kLean96 = 0, kLean160 = 1, kLean256 = 2, kLean128 = 3, kL
 //   cs = 120, 500 blocks (M <= 137):    .099 / .107 / .109 / .092 / .107
 //   cs =  60, 5k blocks (M <=  77):     0.24 / 0.32 / 0.42 / 0.26 / 0.37
 //   cs =  80, 10k blocks (M <=  97):    0.74 / 0.81 / 1.08 / 0.73 / 1.01
-//   cs = 120, 20k blocks (M <= 137):    2.54 / 2.73 / 3.41 / 2.45 / 3.31
+//   cs = 120, 20k blocks (M <= 137):    2.49 / 2.73 / 3.48 / 2.42 / 3.29
 //   cs = 160, 10k blocks (M <= 177):    2.59 / 2.33 / 2.58 / 2.22 / 2.76
-//   cs = 200, 100k blocks (M <= 217):   47.8 / 34.6 / 37.2 / 38.1 / 42.9
+//   cs = 200, 100k blocks (M <= 217):   46.7 / 33.7 / 37.3 / 37.4 / 42.2
 //   cs = 240, 10k blocks (M <= 257):    7.28 / 5.21 / 5.26 / 5.77 / 6.25
-//   cs = 300, 1.5k blocks (M <= 322):   2.91 / 1.87 / 1.45 / 2.09 / 1.86
+//   cs = 300, 1.5k blocks (M <= 322):   2.88 / 1.84 / 1.43 / 2.09 / 1.84
 //   cs = 300, 20k blocks (M <= 317):    33.4 / 20.9 / 17.1 / 24.1 / 20.8
 // nu = 0.8:
 //   cs =  60, 5k blocks (M <=  77):     0.35 / 0.42 / 0.53 / 0.36 / 0.44
 //   cs =  80, 10k blocks (M <=  97):    0.95 / 1.06 / 1.34 / 0.93 / 1.13
 //   cs = 120, 10k blocks (M <= 137):    1.76 / 1.70 / 2.05 / 1.59 / 1.96
 //   cs = 200, 10k blocks (M <= 217):    5.37 / 4.29 / 4.60 / 4.53 / 4.84
-//   cs = 300, 20k blocks (M <= 317):    36.1 / 23.8 / 21.0 / 27.1 / 23.5
+//   cs = 300, 20k blocks (M <= 317):    35.7 / 23.8 / 20.8 / 26.8 / 23.3
 // space-time:
 //   cs =  30, 2.5k blocks (M <=  44):   0.20 / 0.21 / 0.23 / 0.19 / 0.26
 //   cs =  47, 250 blocks (M <=  61):    .099 / .062 / .052 / .073 / .063
@@ -799,13 +799,20 @@ __device__ __forceinline__ void process_block_lean(const LlhArgs &a, const Mater
         const int rend = (warp == 0) ? rw0 : Mp;
         for (int r = (warp == 0) ? rs0 + lane : rw0 + tid - 32; r < rend; r += (warp == 0) ? 32 : kT - 32)
             solve_row(sh, cur + (r - k0) * 16, r);
-        __syncthreads();
-        // Panel p to the slab; panel p+1 takes panel p's update.
-        {
-            double *pg = slab + big_panel_base(p, Mp);
+        if (warp == 0) {
+            // Its rows to the slab while the others still update (after the
+            // barrier, by all warps: n = 1M, cs = 200 34.6 against 33.7 ms).
+            __syncwarp();
             const double2 *s2 = reinterpret_cast<const double2 *>(cur);
-            double2 *g2 = reinterpret_cast<double2 *>(pg);
-            for (int e = tid; e < (Mp - k0) * 8; e += kT) g2[e] = s2[e];
+            double2 *g2 = reinterpret_cast<double2 *>(slab + big_panel_base(p, Mp));
+            for (int e = lane; e < (rw0 - k0) * 8; e += 32) g2[e] = s2[e];
+        }
+        __syncthreads();
+        // The other rows to the slab; panel p+1 takes panel p's update.
+        if (rw0 < Mp) {
+            const double2 *s2 = reinterpret_cast<const double2 *>(cur);
+            double2 *g2 = reinterpret_cast<double2 *>(slab + big_panel_base(p, Mp));
+            for (int e = (rw0 - k0) * 8 + tid; e < (Mp - k0) * 8; e += kT) g2[e] = s2[e];
         }
         if (kb1 > 0) last_update<NT>(nxt, cur, M, k0, n0);
         __syncthreads();
