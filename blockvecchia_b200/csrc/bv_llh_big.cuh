@@ -132,28 +132,13 @@ __device__ __forceinline__ void update_warps_sync()
     asm volatile("bar.sync 1, %0;" ::"n"(NT - 32) : "memory");
 }
 
-// Entry (i, j) of the augmented system: covariance for i < M (plus the
-// nugget on the diagonal), the observation of point j on row M.  Same
-// argument order and the same nugget addition as the shared-memory path's
-// generation, so the entries are identical.
-template <bool kXYZ3>
-__device__ __forceinline__ double big_entry(const double *X, const double *Y, const double *Z,
-                                            const double *T, int M, int i, int j, const MaternParams &mp)
-{
-    if (i >= M) return Z[j];
-    double c;
-    if constexpr (kXYZ3)
-        c = cov_xyz(X[i], Y[i], T[i], X[j], Y[j], T[j], mp);
-    else
-        c = matern(X[i], Y[i], X[j], Y[j], mp);
-    return (i == j && mp.nugget != 0.0) ? c + mp.nugget : c;
-}
-
 // Column c of a 16-column panel starting at row and column q0, rows
 // [r_begin, Mp) step `rstep`, into dst (local row r - dst_r0, swizzled): the
 // column point is read once and kept in registers; entries above the
-// diagonal and columns beyond the matrix (c >= kbq) are zeros.  The same
-// entries as big_entry.
+// diagonal and columns beyond the matrix (c >= kbq) are zeros.  Entry (i, j)
+// is the covariance for i < M (plus the nugget on the diagonal), with the
+// shared-memory path's argument order and nugget addition, so that the values
+// are identical, and the observation of point j on row M.
 template <bool kXYZ3>
 __device__ __forceinline__ void gen_column(double *dst, int dst_r0, const double *X, const double *Y,
                                            const double *Z, const double *T, int M, int Mp, int q0, int kbq,

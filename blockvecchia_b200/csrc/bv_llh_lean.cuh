@@ -131,7 +131,7 @@ struct TileLane {
 // tile m's rows i0 + m * rstep + r8, columns n0 + 8 nj + 2 c4 + e.  Rows
 // beyond the block and entries above the diagonal are zeros; row M holds the
 // observations; columns beyond the block are unspecified (never used).  The
-// values are those of big_entry for the closed forms (nu = 1/2, 3/2, 5/2),
+// values are those of gen_column for the closed forms (nu = 1/2, 3/2, 5/2),
 // which share the distance and the exponential; the 4 NTILE entries of a lane
 // are independent chains.
 template <int NTILE>

@@ -92,8 +92,8 @@ __global__ void __launch_bounds__(kThreads, 1) llh_fp64_server_kernel(const JobD
 // The multi-CTA streamed kernel's server form: the same task list protocol
 // over the blocks whose two panels fit in shared memory (the rest run the
 // kernel above), NT threads per CTA, MINB CTAs per SM, one global slab per
-// CTA.  Per block the code of the handles' default path (process_block_lean,
-// panel-by-panel generation), so a request's blocks give the bits a handle
+// CTA.  Per block the code of the handles' default path
+// (process_block_lean), so a request's blocks give the bits a handle
 // created with the default schedule gives.
 template <int NT, int MINB, int GEN>
 __global__ void __launch_bounds__(NT, MINB) llh_lean_server_kernel(const JobDesc *descs, const int2 *tasks,
