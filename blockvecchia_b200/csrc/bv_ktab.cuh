@@ -36,14 +36,29 @@ constexpr int kTabEntries = kTabPairs * kTabN;    // double2s of a table
 constexpr int kTabWinOct = 12, kTabWinN = 8 * kTabWinOct;
 constexpr int kTabWinBytes = kTabPairs * kTabWinN * (int)sizeof(double2);
 
-// Region 1's top: the exponent e with 2^e <= (11.3 range dist_scale)^2, or no
-// table where squared distances of that size leave the normal range.
+// Region 1's top: the exponent e with 2^e <= (11.3 range dist_scale)^2.  No
+// table where squared distances of that size leave the normal range, or where
+// matern_general does at the table's lower end (r ~ 1.2e-4): it multiplies
+// con r^nu, both tiny for a large nu, by K_nu(r) < 2^(nu-1) Gamma(nu) r^-nu,
+// and a node that is not finite would take its whole interval with it,
+// entries of larger r among them (at nu = 60 the entries from r = 3.1e-4 to
+// 3.2e-4).  At sigma2 = 1 the line is at nu ~ 55.
 inline void ktab_prepare(MaternParams &p)
 {
-    const double top = 11.313708498984761 * p.range * p.dist_scale;
+    p.kt_on = 0;
+    p.kt_e1 = 0;
+    const double scale = p.range * p.dist_scale;
+    const double top = 11.313708498984761 * scale;
     const double s = top * top;
-    p.kt_on = (s > 1e-250 && s < 1e250) ? 1 : 0;
-    p.kt_e1 = p.kt_on ? std::ilogb(s) : 0;
+    if (!(s > 1e-250 && s < 1e250)) return;
+    const int e1 = std::ilogb(s);
+    const double log_r = 0.5 * 0.6931471805599453 * (e1 - kTabOct1) - std::log(scale);
+    const double log_pow = p.nu * log_r;                                                  // r^nu
+    const double log_k = (p.nu - 1.0) * 0.6931471805599453 + std::lgamma(p.nu) - log_pow;  // above K_nu(r)
+    if (log_pow < -690.0 || log_k > 700.0) return;
+    if (p.sigma2 != 0.0 && std::log(std::fabs(p.con)) + log_pow < -690.0) return;
+    p.kt_on = 1;
+    p.kt_e1 = e1;
 }
 
 // Coefficients of the Chebyshev polynomials T_0 .. T_kTabDeg: T[k][j] t^j.
