@@ -35,7 +35,8 @@
 // same operations as in a scan of the whole prefix, and S does not depend on
 // the order of the candidates.  A scan of the whole prefix (5e10 keys at 1M
 // points and 100k blocks) remains for great-circle keys, small layouts and
-// prefixes, and windows that would hold more points than the prefix.
+// prefixes, and blocks whose windows would hold more points in all than the
+// prefix (3-D keys: than half of it).
 // A block whose ties at the k-th key overflow the warp's buffer (hundreds of
 // exactly repeated locations at one distance) is listed and redone by
 // knn_heavy_kernel: one CTA, keys recomputed on every pass instead of
@@ -445,6 +446,15 @@ __global__ void __launch_bounds__(kKnnWarps * 32) knn_kernel(KnnArgs a)
             const int gx = grid_cell1(cx, g.x0, g.ihx, g.nx), gy = grid_cell1(cy, g.y0, g.ihy, g.ny);
             // Locations that should hold the set: 1.6 k earlier ones.
             const double want = 1.6 * (double)k * ((double)a.n / (double)P);
+            // The first window is scanned if it holds less than the prefix.
+            // Further ones while all of them hold less than it, or for a 3-D
+            // key, whose window may tell nothing about the third coordinate,
+            // less than half of it.  Kernel ms, 300k points, 30k blocks, cs =
+            // 100, third coordinates over 1 / 30 / 1,000 times the plane's
+            // extent: 4.1 / 19.9 / 39.1 (prefixes alone 27.4, windows of up to the prefix
+            // each 4.1 / 19.5 / 74.0).
+            const int further = (kGeo == kGeo3D) ? P / 2 : P;
+            int scanned = 0;
             int r = 1;
             for (whole = false;;) {
                 // The smallest window (from the present one on) with as many.
@@ -461,10 +471,11 @@ __global__ void __launch_bounds__(kKnnWarps * 32) knn_kernel(KnnArgs a)
                     if ((double)held >= want || held >= P || held == a.n) break;
                     r += (r + 2) / 3;
                 }
-                if (held >= P) {  // no fewer than the prefix: scan that
+                if (held >= (scanned > 0 ? further - scanned : P)) {
                     whole = true;
                     break;
                 }
+                scanned += held;
                 count = 0;
                 for (int row = y0; row <= y1 && !overflow; ++row) {
                     const int j1 = a.start[row * g.nx + x1 + 1];
