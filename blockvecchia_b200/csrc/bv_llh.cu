@@ -124,9 +124,11 @@ struct LeanVariant {
 #define BV_LEAN(NT, MINB)                                                                          \
     {{llh_lean_kernel_t<NT, MINB, kGenClosed>, llh_lean_kernel_t<NT, MINB, kGenGeneral>,          \
       llh_lean_kernel_t<NT, MINB, kGenXYZ>}, NT}
-// In the order of LeanShape, and one more for the tuner; the last entry is the
-// one-warp kernel where it applies (warp_variant).  All give the same bits, so
-// bv_opts.tune may pick any.
+// In the order of LeanShape, and one more for the tuner: 256 x 1 is up to 2%
+// faster than 256 x 2 for a few blocks of M ~ 520 and more (cs = 500, 2k blocks
+// 8.69 against 8.83 ms; cs = 700, 150 blocks 3.47 / 3.48) and slower below (cs
+// = 300, 20k blocks 24.6 / 17.0).  In its place the one-warp kernel, where that
+// applies (warp_variant).  All give the same bits, so bv_opts.tune may pick any.
 static const LeanVariant kLeanVariants[] = {
     BV_LEAN(96, 5), BV_LEAN(160, 3), BV_LEAN(256, 2), BV_LEAN(128, 4), BV_LEAN(160, 2), BV_LEAN(256, 1),
 };
@@ -205,11 +207,14 @@ struct bv_handle {
     int lean_max_m = 0;             // blocks with M <= this run the multi-CTA streamed kernel
     int streamed_blocks = 0;        // of the owned blocks, how many that is
     bool mixed_lean = false;        // mixed path: the FP64 pass runs the streamed kernel (last launch)
-    // The streamed launch's order positions and largest M, its CTA size
-    // (kLeanVariants index; -1: from the table), and the tuner's record.
-    int lean_begin = 0, lean_end = 0, lean_m = 0, lean_choice = -1;
-    bool tuned = false;
-    double tune_ms[kNumLean] = {};
+    // The streamed launch's place among the launches (-1: none), its order
+    // positions and largest M, and per kind of evaluation (closed-form nu,
+    // general nu; with a third coordinate only the first) its variant
+    // (kLeanVariants index; -1: from the table) and the tuner's record.
+    int lean_index = -1, lean_begin = 0, lean_end = 0, lean_m = 0;
+    int lean_choice[2] = {-1, -1};
+    bool tuned[2] = {false, false};
+    double tune_ms[2][kNumLean] = {};
     MaternParams *d_mp = nullptr;
     double2 *d_ktab = nullptr;  // the general-nu table (bv_ktab.cuh)
     MixedWork mixed;  // mixed-precision scratch (bv_llh_mixed.cuh)
@@ -452,6 +457,7 @@ static int order_m(const bv_handle *h, int t)
 // largest block has M = max_m.
 static int plan_lean_launch(bv_handle *h, const cudaDeviceProp &prop, int begin, int end, int max_m)
 {
+    h->lean_index = (int)h->launches.size();
     h->lean_begin = begin;
     h->lean_end = end;
     h->lean_m = max_m;
@@ -462,7 +468,8 @@ static int plan_lean_launch(bv_handle *h, const cudaDeviceProp &prop, int begin,
     for (int g = 0; g < 2; ++g) {
         bv_handle::Kernel &k = ln.k[g];
         const int gen = h->nz ? kGenXYZ : g;
-        k.variant = h->lean_choice >= 0 ? h->lean_choice : lean_variant(gen, max_m, (size_t)(end - begin));
+        const int choice = h->lean_choice[h->nz ? 0 : g];
+        k.variant = choice >= 0 ? choice : lean_variant(gen, max_m, (size_t)(end - begin));
         const LeanVariant &v = kLeanVariants[k.variant];
         const bool warp = k.variant == kNumLean - 1 && warp_variant(gen, max_m);
         k.fn = warp ? llh_warp_kernel : v.kernel[gen];
@@ -631,13 +638,9 @@ static cudaError_t record_timing(cudaEvent_t ev, cudaStream_t s)
 
 static int capture_graph(bv_handle *h);
 
-// Kinds of evaluation that differ in their launches.
-static int graph_kinds(const bv_handle *h)
-{
-    for (const bv_handle::Launch &ln : h->launches)
-        if (ln.k[0].fn != ln.k[1].fn) return 2;
-    return 1;
-}
+// Kinds of evaluation that differ in their launches: the streamed kernel on
+// 2-D locations has one for the closed forms and one for a general nu.
+static int graph_kinds(const bv_handle *h) { return (h->lean_index >= 0 && !h->nz) ? 2 : 1; }
 
 static int eval_kind(const bv_handle *h)
 {
@@ -967,10 +970,7 @@ static int fill_params(bv_handle *h, const double *theta)
     return BV_OK;
 }
 
-// One evaluation of each kind captured into the handle's graphs (replacing
-// any earlier).  Without a streamed launch, or with a third coordinate, both
-// kinds run the same kernels and share the first graph.
-static int capture_graph(bv_handle *h)
+static void drop_graphs(bv_handle *h)
 {
     for (int g = 0; g < 2; ++g) {
         if (h->gexec[g]) cudaGraphExecDestroy(h->gexec[g]);
@@ -978,6 +978,14 @@ static int capture_graph(bv_handle *h)
         h->gexec[g] = nullptr;
         h->graph[g] = nullptr;
     }
+}
+
+// One evaluation of each kind captured into the handle's graphs (replacing
+// any earlier).  Without a streamed launch, or with a third coordinate, both
+// kinds run the same kernels and share the first graph.
+static int capture_graph(bv_handle *h)
+{
+    drop_graphs(h);
     for (int g = 0; g < graph_kinds(h); ++g) {
         BV_CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
         const int erc = enqueue_eval(h, h->stream, g);
@@ -994,47 +1002,54 @@ static int capture_graph(bv_handle *h)
     return BV_OK;
 }
 
-// The streamed launch (always the last one planned) again, with CTA size vi.
-static int replan_lean(bv_handle *h, int vi)
+// The streamed launch (always the last one planned) again, with variant vi for
+// evaluations of one kind.
+static int replan_lean(bv_handle *h, int kind, int vi)
 {
     cudaDeviceProp prop;
     BV_CUDA_TRY(cudaGetDeviceProperties(&prop, h->device));
-    h->launches.pop_back();
+    drop_graphs(h);  // they name the slab
+    h->launches.resize((size_t)h->lean_index);
     cudaFree(h->d_slab_lean);
     h->d_slab_lean = nullptr;
-    h->lean_choice = vi;
+    h->lean_choice[kind] = vi;
     return plan_lean_launch(h, prop, h->lean_begin, h->lean_end, h->lean_m);
 }
 
-// bv_opts.tune: on the first evaluation, time the streamed kernel at every
-// CTA size (twice each, the faster kept) and keep the fastest.  The sizes
-// give the same bits, so the evaluation's value does not depend on it.
-static int tune_lean(bv_handle *h)
+// bv_opts.tune: on the first evaluation of each kind, time the streamed
+// kernel's variants (twice each, the faster kept) and keep the fastest for
+// that kind: the two kinds' kernels differ in registers, shared memory and
+// speed, and the last variant is the one-warp kernel for one of them only
+// (30k blocks of M = 31 tuned at nu = 0.5 took 2.04 ms at nu = 0.8 on the
+// variant kept for both, .70 on the table's).  The variants give the same
+// bits, so an evaluation's value does not depend on it.
+static int tune_lean(bv_handle *h, int kind)
 {
-    h->tuned = true;
     int best = 0;
     double best_ms = 1e300;
     for (int vi = 0; vi < kNumLean; ++vi) {
-        int rc = replan_lean(h, vi);
+        int rc = replan_lean(h, kind, vi);
         if (rc) return rc;
         double t = 1e300;
         for (int rep = 0; rep < 2; ++rep) {
-            rc = enqueue_eval(h, h->stream, eval_kind(h));
+            rc = enqueue_eval(h, h->stream, kind);
             if (rc) return rc;
             BV_CUDA_TRY(cudaStreamSynchronize(h->stream));
             float kms = 0.f;
             BV_CUDA_TRY(cudaEventElapsedTime(&kms, h->evk0, h->evk1));
             t = std::min(t, (double)kms);
         }
-        h->tune_ms[vi] = t;
+        h->tune_ms[kind][vi] = t;
         if (t < best_ms) {
             best_ms = t;
             best = vi;
         }
     }
-    int rc = replan_lean(h, best);
+    int rc = replan_lean(h, kind, best);
     if (rc) return rc;
-    return h->opts.use_graph ? capture_graph(h) : BV_OK;
+    if (h->opts.use_graph && (rc = capture_graph(h))) return rc;
+    h->tuned[kind] = true;
+    return BV_OK;
 }
 
 static int eval_locked(bv_handle *h, const double *theta, double *llk)
@@ -1042,12 +1057,17 @@ static int eval_locked(bv_handle *h, const double *theta, double *llk)
     int rc = fill_params(h, theta);
     if (rc) return rc;
     BV_CUDA_TRY(cudaSetDevice(h->device));
-    if (h->opts.tune && !h->tuned && h->streamed_blocks > 0 && h->opts.precision == BV_PREC_FP64) {
-        rc = tune_lean(h);
+    const int kind = eval_kind(h);
+    // A tuner that could not allocate left no streamed launch.
+    if (h->lean_index >= 0 && (int)h->launches.size() == h->lean_index) {
+        rc = replan_lean(h, kind, -1);
+        if (rc) return rc;
+    }
+    if (h->opts.tune && !h->tuned[kind] && h->streamed_blocks > 0 && h->opts.precision == BV_PREC_FP64) {
+        rc = tune_lean(h, kind);
         if (rc) return rc;
     }
     BV_CUDA_TRY(cudaEventRecord(h->ev0, h->stream));
-    const int kind = eval_kind(h);
     if (h->gexec[kind]) {
         BV_CUDA_TRY(cudaGraphLaunch(h->gexec[kind], h->stream));
     } else {
@@ -1083,7 +1103,7 @@ static int eval_locked(bv_handle *h, const double *theta, double *llk)
     const bv_handle::Kernel *lk = s.streamed_blocks > 0 ? &h->launches.back().k[kind] : nullptr;
     s.streamed_threads = lk ? lk->threads : 0;
     s.streamed_variant = lk ? lk->variant : -1;
-    for (int i = 0; i < kNumLean; ++i) s.tune_ms[i] = h->tune_ms[i];
+    for (int i = 0; i < kNumLean; ++i) s.tune_ms[i] = h->tune_ms[kind][i];
     s.llk = r.llk;
     double v = r.llk;
     const bool failed = (r.cond_fail + r.schur_fail + r.nonfinite) > 0 || !std::isfinite(v);

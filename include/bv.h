@@ -133,10 +133,12 @@ typedef struct {
                           as the reference allows it for 2-D locations only. */
     int tune;          /* 0 (default): the streamed kernel's variant from a
                           measured table by the launch's largest block.  1:
-                          the first evaluation times every variant on this
-                          layout and the handle keeps the fastest (all give
-                          the same bits, so results do not depend on the
-                          choice); bv_get_status reports the times.        */
+                          the first evaluation at a closed-form nu (1/2, 3/2,
+                          5/2) and the first at any other time every variant
+                          on this layout, and the handle keeps the fastest
+                          for each (all give the same bits, so results do not
+                          depend on the choice); bv_get_status reports the
+                          times.                                           */
     int mixed_fp32;    /* BV_PREC_MIXED only.  0 (default): every block on the
                           FP64 path (its values exactly): on B200 the FP32
                           factor + FP64 refinement kernel took 4.8-6.3x the
@@ -171,12 +173,12 @@ typedef struct {
                             0 for the mixed path                             */
     int streamed_threads; /* threads per CTA of that kernel (0: none)       */
     int streamed_variant; /* its variant, an index into tune_ms             */
-    double tune_ms[6];   /* with bv_opts.tune: the streamed kernel's time on
-                            the first evaluation per variant: 96 threads x 5
-                            CTAs per SM, 160 x 3, 256 x 2, 128 x 4, 160 x 2
-                            and 256 x 1 (blocks up to M = 48 at a closed-form
-                            nu one per warp in the last's place; 0 where not
-                            timed)                                           */
+    double tune_ms[6];   /* with bv_opts.tune: the streamed kernel's time per
+                            variant, as the tuner took it for the last
+                            evaluation's kind of nu: 96 threads x 5 CTAs per
+                            SM, 160 x 3, 256 x 2, 128 x 4, 160 x 2 and 256 x 1
+                            (blocks up to M = 48 at a closed-form nu one per
+                            warp in the last's place; 0 where not timed)     */
 } bv_status;
 
 typedef struct bv_handle bv_handle;
