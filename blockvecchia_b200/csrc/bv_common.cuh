@@ -34,12 +34,15 @@ int fp64_limits(int device, size_t *avail, int *small_m, int *big_m, int nz = 0)
 // algorithm.  Block 0 is unconditioned (M = bs).
 bool use_big_path(const int *batchNum, int bc, int cs, int small_m, int big_m, int sm_count);
 
+// The error is reported here and now: it is taken off the thread's record,
+// where the next kernel launch's check would find it again.
 #define BV_CUDA_TRY(expr)                                                          \
     do {                                                                           \
         cudaError_t _e = (expr);                                                   \
         if (_e != cudaSuccess) {                                                   \
             ::bv::set_error("%s failed at %s:%d: %s", #expr, __FILE__, __LINE__,   \
                             cudaGetErrorString(_e));                               \
+            cudaGetLastError();                                                    \
             return BV_E_CUDA;                                                      \
         }                                                                          \
     } while (0)

@@ -451,8 +451,8 @@ __global__ void __launch_bounds__(kKnnWarps * 32) knn_kernel(KnnArgs a)
             // key, whose window may tell nothing about the third coordinate,
             // less than half of it.  Kernel ms, 300k points, 30k blocks, cs =
             // 100, third coordinates over 1 / 30 / 1,000 times the plane's
-            // extent: 4.1 / 19.9 / 39.1 (prefixes alone 27.4, windows of up to the prefix
-            // each 4.1 / 19.5 / 74.0).
+            // extent: 4.1 / 19.9 / 39.1 (prefixes alone 27.4, windows of up
+            // to the prefix each 4.1 / 19.5 / 74.0).
             const int further = (kGeo == kGeo3D) ? P / 2 : P;
             int scanned = 0;
             int r = 1;
@@ -836,6 +836,7 @@ int knn_device(const double *d_x, const double *d_y, const double *d_z, int n, i
     int rc = BV_OK;
     auto fail = [&](cudaError_t e, const char *what) {
         set_error("bv_knn: %s: %s", what, cudaGetErrorString(e));
+        cudaGetLastError();
         rc = BV_E_CUDA;
     };
     cudaError_t e;
@@ -1045,6 +1046,7 @@ static int knn_host(const double *x, const double *y, const double *z, int n, in
         if ((e = cudaMalloc(&d_x, nd * sizeof(double) + ((size_t)bc + 1) * sizeof(int))) ||
             (e = cudaMalloc(&d_knn, sizeof(int) * (size_t)bc * cs))) {
             set_error("bv_knn: cudaMalloc: %s", cudaGetErrorString(e));
+            cudaGetLastError();
             rc = (e == cudaErrorMemoryAllocation) ? BV_E_NOMEM : BV_E_CUDA;
             break;
         }
@@ -1056,6 +1058,7 @@ static int knn_host(const double *x, const double *y, const double *z, int n, in
             (z && (e = cudaMemcpyAsync(d_z, z, sizeof(double) * n, cudaMemcpyHostToDevice, s))) ||
             (e = cudaMemcpyAsync(d_acc, batchNumAccum, sizeof(int) * (bc + 1), cudaMemcpyHostToDevice, s))) {
             set_error("bv_knn: copy: %s", cudaGetErrorString(e));
+            cudaGetLastError();
             rc = BV_E_CUDA;
             break;
         }
@@ -1073,6 +1076,7 @@ static int knn_host(const double *x, const double *y, const double *z, int n, in
             if ((e = cudaMemcpyAsync(knn_idx + (size_t)e0 * cs, d_knn + (size_t)e0 * cs,
                                      sizeof(int) * (size_t)(e1 - e0) * cs, cudaMemcpyDeviceToHost, s))) {
                 set_error("bv_knn: copy back: %s", cudaGetErrorString(e));
+                cudaGetLastError();
                 rc = BV_E_CUDA;
                 break;
             }
@@ -1081,6 +1085,7 @@ static int knn_host(const double *x, const double *y, const double *z, int n, in
         if (rc) break;
         if ((e = cudaStreamSynchronize(s))) {
             set_error("bv_knn: copy back: %s", cudaGetErrorString(e));
+            cudaGetLastError();
             rc = BV_E_CUDA;
         }
     } while (0);

@@ -774,6 +774,7 @@ extern "C" int bv_create(const bv_layout *L, const bv_opts *opts, bv_handle **ou
         cudaError_t _e = (expr);                                                         \
         if (_e != cudaSuccess) {                                                         \
             set_error("%s: %s", #expr, cudaGetErrorString(_e));                          \
+            cudaGetLastError();                                                          \
             handle_free(h);                                                              \
             return (_e == cudaErrorMemoryAllocation) ? BV_E_NOMEM : BV_E_CUDA;           \
         }                                                                                \
