@@ -246,11 +246,14 @@ struct bv_handle {
     cudaStream_t stream = nullptr;
     cudaGraph_t graph[2] = {nullptr, nullptr};  // closed-form nu, general nu
     cudaGraphExec_t gexec[2] = {nullptr, nullptr};
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr, evk0 = nullptr, evk1 = nullptr;
+    // Around the evaluation, two pairs in turn (finish_times), and around its
+    // blocks' kernels.
+    cudaEvent_t ev[2][2] = {}, evk0 = nullptr, evk1 = nullptr;
     cudaStream_t own_stream = nullptr;  // the handle's stream; `stream` may be a caller's
     // status
     bv_status status{};
-    bool timed = false;  // status.device_ms / kernel_ms are to be read from the events
+    bool timed = false;  // the last evaluation's times are still in ev[ev_last], evk0, evk1
+    int ev_last = 0;
     int iterations = 0;
 };
 
@@ -264,8 +267,9 @@ static void handle_free(bv_handle *h)
         if (h->gexec[g]) cudaGraphExecDestroy(h->gexec[g]);
         if (h->graph[g]) cudaGraphDestroy(h->graph[g]);
     }
-    if (h->ev0) cudaEventDestroy(h->ev0);
-    if (h->ev1) cudaEventDestroy(h->ev1);
+    for (auto &pair : h->ev)
+        for (cudaEvent_t e : pair)
+            if (e) cudaEventDestroy(e);
     if (h->evk0) cudaEventDestroy(h->evk0);
     if (h->evk1) cudaEventDestroy(h->evk1);
     if (h->own_stream) cudaStreamDestroy(h->own_stream);
@@ -844,8 +848,8 @@ extern "C" int bv_create(const bv_layout *L, const bv_opts *opts, bv_handle **ou
 
     BV_CUDA_H(cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking));
     h->stream = h->own_stream;
-    BV_CUDA_H(cudaEventCreate(&h->ev0));
-    BV_CUDA_H(cudaEventCreate(&h->ev1));
+    for (auto &pair : h->ev)
+        for (cudaEvent_t &e : pair) BV_CUDA_H(cudaEventCreate(&e));
     BV_CUDA_H(cudaEventCreate(&h->evk0));
     BV_CUDA_H(cudaEventCreate(&h->evk1));
     const size_t n = h->n, bc = h->bc, cs = h->cs;
@@ -1053,6 +1057,26 @@ static int tune_lean(bv_handle *h, int kind)
     return BV_OK;
 }
 
+// The last evaluation's times from its events into the status, where they are
+// still to be read: by bv_get_status, and before those events are recorded
+// again otherwise than by a whole evaluation.  (Read in every evaluation they
+// cost a 2k-point one 5.6 of its 60 us.)  The next evaluation records the other
+// pair of ev; one from the graph records evk0 and evk1 only once it has been
+// launched, so that one refused before that leaves these times as they were.
+static void finish_times(bv_handle *h)
+{
+    if (!h->timed) return;
+    h->timed = false;
+    float ms = 0.f, kms = 0.f;
+    if (cudaEventElapsedTime(&ms, h->ev[h->ev_last][0], h->ev[h->ev_last][1]) != cudaSuccess ||
+        cudaEventElapsedTime(&kms, h->evk0, h->evk1) != cudaSuccess) {
+        cudaGetLastError();
+        ms = kms = 0.f;
+    }
+    h->status.device_ms = ms;
+    h->status.kernel_ms = kms;
+}
+
 static int eval_locked(bv_handle *h, const double *theta, double *llk)
 {
     int rc = fill_params(h, theta);
@@ -1065,19 +1089,23 @@ static int eval_locked(bv_handle *h, const double *theta, double *llk)
         if (rc) return rc;
     }
     if (h->opts.tune && !h->tuned[kind] && h->streamed_blocks > 0 && h->opts.precision == BV_PREC_FP64) {
+        finish_times(h);
         rc = tune_lean(h, kind);
         if (rc) return rc;
     }
-    BV_CUDA_TRY(cudaEventRecord(h->ev0, h->stream));
+    if (!h->gexec[kind]) finish_times(h);
+    const int pair = h->ev_last ^ 1;
+    BV_CUDA_TRY(cudaEventRecord(h->ev[pair][0], h->stream));
     if (h->gexec[kind]) {
         BV_CUDA_TRY(cudaGraphLaunch(h->gexec[kind], h->stream));
     } else {
         rc = enqueue_eval(h, h->stream, kind);
         if (rc) return rc;
     }
-    BV_CUDA_TRY(cudaEventRecord(h->ev1, h->stream));
+    BV_CUDA_TRY(cudaEventRecord(h->ev[pair][1], h->stream));
     BV_CUDA_TRY(cudaStreamSynchronize(h->stream));
     h->timed = true;
+    h->ev_last = pair;
     const EvalResult r = *h->h_res;
     bv_status &s = h->status;
     s.blocks = h->owned;
@@ -1208,14 +1236,7 @@ extern "C" int bv_get_status(bv_handle *h, bv_status *st)
 {
     if (!h || !st) return BV_E_INVALID;
     std::lock_guard<std::mutex> lk(h->mu);
-    if (h->timed) {  // the last evaluation's events have completed
-        float ms = 0.f, kms = 0.f;
-        cudaEventElapsedTime(&ms, h->ev0, h->ev1);
-        cudaEventElapsedTime(&kms, h->evk0, h->evk1);
-        h->status.device_ms = ms;
-        h->status.kernel_ms = kms;
-        h->timed = false;
-    }
+    finish_times(h);
     *st = h->status;
     return BV_OK;
 }

@@ -161,7 +161,8 @@ typedef struct {
     int nonfinite;       /* blocks whose contribution was not finite         */
     unsigned flags_or;   /* OR of BV_ST_* over all blocks                    */
     double llk;          /* last log-likelihood (before the failure policy)  */
-    double device_ms;    /* device time of the last evaluation               */
+    double device_ms;    /* device time of the last evaluation that gave a
+                            value                                            */
     double kernel_ms;    /* of which the fused per-block kernel(s)            */
     int failed;          /* blocks with a failed pivot in either factor
                             (cond_fail and schur_fail may count one block
