@@ -1,5 +1,7 @@
 """Where a block's search through the grid of bv_knn ends: a third coordinate
-that dwarfs the plane.  Indices and order against findNearestPoints, bit-exact."""
+that dwarfs the plane, centroids beyond every side and corner of the
+locations, locations far from the origin, keys beyond the double range.
+Indices and order against findNearestPoints, bit-exact."""
 import time
 
 import numpy as np
@@ -55,3 +57,65 @@ def test_deep_third_coordinate_cost(bvlib):
             t.append(time.perf_counter() - t0)
         best.append(min(t))
     assert best[0] <= 1.95 * best[1], best
+
+
+def _planar(n, cs, g, x, y):
+    bn = np.array([cs + 5] + [5] * ((n - cs - 5) // 5), np.int32)
+    bn[-1] += n - int(bn.sum())
+    acc = np.concatenate([[0], np.cumsum(bn)]).astype(np.int32)
+    return bn, acc, x[acc[:-1]].copy(), y[acc[:-1]].copy()
+
+
+@pytest.mark.parametrize("kind", ["uniform", "clusters"])
+@pytest.mark.parametrize("cs", [7, 60])
+def test_centroids_outside(bvlib, oracle, kind, cs):
+    """Centroids of blocks that search the grid (2,048 earlier locations and
+    more) beyond each side and corner: just outside, by a third of the extent
+    and far away, and the opposite way round at positions along the sides."""
+    g = np.random.default_rng(cs)
+    n = 9000
+    x, y = g.random(n), g.random(n)
+    if kind == "clusters":
+        c = g.integers(0, 6, n)
+        x = g.random(6)[c] + 0.01 * g.standard_normal(n)
+        y = g.random(6)[c] + 0.01 * g.standard_normal(n)
+    bn, acc, cx, cy = _planar(n, cs, g, x, y)
+    late = np.flatnonzero(acc[:-1] >= 2048)
+    moved = g.permutation(late)[:160]
+    for t, b in enumerate(moved):
+        sx, sy = ((-1, 0), (1, 0), (0, -1), (0, 1), (-1, -1), (-1, 1), (1, -1), (1, 1))[t % 8]
+        h = (1e-9, 1e-3, 0.3, 40.0, 1e7)[t // 8 % 5]
+        if sx:
+            cx[b] = x.max() + h if sx > 0 else x.min() - h
+        if sy:
+            cy[b] = y.max() + h if sy > 0 else y.min() - h
+    assert np.all(acc[moved] >= 2048)
+    L = bvlib.Layout(bn, acc, x, y, np.zeros(n), cs, cx, cy)
+    assert np.array_equal(bvlib.knn(L), oracle.knn_all_fast(x, y, cs, acc, cx, cy))
+
+
+@pytest.mark.parametrize("cs", [3, 20, 60])
+@pytest.mark.parametrize("e", [41, 44])
+def test_far_from_the_origin(bvlib, oracle, cs, e):
+    """A unit square at 2^41 (coordinates are multiples of 2^-11, a thirtieth
+    of a cell) and 2^44 (a quarter): a window's sides are not representable as
+    coordinates."""
+    g = np.random.default_rng(cs + e)
+    n = 16000
+    x, y = g.random(n) + 2.0 ** e, g.random(n) - 2.0 ** e
+    bn, acc, cx, cy = _planar(n, cs, g, x, y)
+    L = bvlib.Layout(bn, acc, x, y, np.zeros(n), cs, cx, cy)
+    assert np.array_equal(bvlib.knn(L), oracle.knn_all_fast(x, y, cs, acc, cx, cy))
+
+
+def test_keys_beyond_the_double_range(bvlib, oracle):
+    """Squared distances that overflow tie at infinity: a third of the
+    locations 1e200 away, and some centroids between."""
+    g = np.random.default_rng(2)
+    n, cs = 6000, 40
+    x, y = g.random(n), g.random(n)
+    x[g.permutation(n)[:n // 3]] += 1e200
+    bn, acc, cx, cy = _planar(n, cs, g, x, y)
+    cx[g.permutation(np.flatnonzero(acc[:-1] >= 2048))[:5]] = 5e199
+    L = bvlib.Layout(bn, acc, x, y, np.zeros(n), cs, cx, cy)
+    assert np.array_equal(bvlib.knn(L), oracle.knn_all_fast(x, y, cs, acc, cx, cy))
