@@ -96,7 +96,7 @@ struct KnnGrid {
 constexpr int kGridOcc = 4;         // mean locations per cell
 constexpr int kGridMinN = 4096;     // smaller layouts scan the prefix
 constexpr int kGridMinPrefix = 2048;  // and so do the first blocks of larger ones
-constexpr int kBoxCtas = 296, kBoxThreads = 256;
+constexpr int kBoxCtas = 296, kBoxThreads = 256;  // partial bounding boxes, each strided over the locations
 
 __device__ __forceinline__ int grid_cell1(double v, double v0, double ih, int n)
 {
@@ -908,6 +908,9 @@ int knn_device(const double *d_x, const double *d_y, const double *d_z, int n, i
         ka.nlist = (int)list.size();
         ka.grid = nullptr;
         ka.n = n;
+        int dev = 0, sms = 0, occ = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (use_grid) {
             double *sx = d_grid, *sy = sx + n, *sz = sy + n;
             double *part = d_z ? sz + n : sz;
@@ -920,7 +923,7 @@ int knn_device(const double *d_x, const double *d_y, const double *d_z, int n, i
             }
             knn_box_kernel<<<kBoxCtas, kBoxThreads, 0, s>>>(d_x, d_y, n, part);
             knn_grid_kernel<<<1, 32, 0, s>>>(part, ncell, grid);
-            const int gb = std::min((n + 255) / 256, 148 * 8);
+            const int gb = std::min((n + 255) / 256, std::max(1, sms) * 8);
             knn_cells_kernel<false><<<gb, 256, 0, s>>>(d_x, d_y, d_z, n, grid, cells, sx, sy, sz, sidx);
             knn_scan_kernel<<<1, 1024, 0, s>>>(cells, start, ncell);
             knn_cells_kernel<true><<<gb, 256, 0, s>>>(d_x, d_y, d_z, n, grid, cells, sx, sy, sz, sidx);
@@ -940,9 +943,6 @@ int knn_device(const double *d_x, const double *d_y, const double *d_z, int n, i
             fail(e, "attribute");
             break;
         }
-        int dev = 0, sms = 0, occ = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kKnnWarps * 32, smem);
         if (occ < 1) occ = 1;
         int grid = sms * occ;

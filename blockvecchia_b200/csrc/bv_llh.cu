@@ -134,12 +134,12 @@ static const LeanVariant kLeanVariants[] = {
 };
 constexpr int kNumLean = (int)(sizeof(kLeanVariants) / sizeof(kLeanVariants[0]));
 static bool warp_variant(int gen, int max_m) { return gen == kGenClosed && max_m <= kWarpMaxM; }
-static int lean_variant(int gen, int max_m, size_t blocks)
+static int lean_variant(int gen, int max_m, size_t blocks, int sms)
 {
-    // A launch that fills the SMs with warps; 500 blocks (cs = 20) take .017 ms
-    // on 96-thread CTAs and .021 one per warp.
-    if (warp_variant(gen, max_m) && blocks >= 4 * 148) return kNumLean - 1;
-    return lean_table(gen, max_m, blocks);
+    // A launch with a block for every sub-partition; 500 blocks (cs = 20) take
+    // .017 ms on 96-thread CTAs and .021 one per warp.
+    if (warp_variant(gen, max_m) && blocks >= 4 * (size_t)sms) return kNumLean - 1;
+    return lean_table(gen, max_m, blocks, sms);
 }
 
 __global__ void __launch_bounds__(kTabThreads) ktab_kernel(const MaternParams *mp, double2 *tab)
@@ -473,7 +473,8 @@ static int plan_lean_launch(bv_handle *h, const cudaDeviceProp &prop, int begin,
         bv_handle::Kernel &k = ln.k[g];
         const int gen = h->nz ? kGenXYZ : g;
         const int choice = h->lean_choice[h->nz ? 0 : g];
-        k.variant = choice >= 0 ? choice : lean_variant(gen, max_m, (size_t)(end - begin));
+        k.variant = choice >= 0 ? choice
+                                : lean_variant(gen, max_m, (size_t)(end - begin), prop.multiProcessorCount);
         const LeanVariant &v = kLeanVariants[k.variant];
         const bool warp = k.variant == kNumLean - 1 && warp_variant(gen, max_m);
         k.fn = warp ? llh_warp_kernel : v.kernel[gen];

@@ -60,7 +60,7 @@ enum LeanShape : int { kLean96 = 0, kLean160 = 1, kLean256 = 2, kLean128 = 3, kL
 // has too few tiles for more than two update warps; a launch of at most two
 // blocks per SM wants each block short.  Entries generated through shared
 // memory (a third coordinate) are a larger share of the update warps' work.
-// Kernel ms at 96 x 5 / 160 x 3 / 256 x 2 / 128 x 4 / 160 x 2:
+// Kernel ms on 148 SMs at 96 x 5 / 160 x 3 / 256 x 2 / 128 x 4 / 160 x 2:
 //   cs =  60, 150 blocks (M <=  82):    .041 / .036 / .034 / .036 / .031
 //   cs = 120, 300 blocks (M <= 137):    .086 / .064 / .064 / .070 / .061
 //   cs = 120, 500 blocks (M <= 137):    .099 / .107 / .109 / .092 / .107
@@ -85,9 +85,9 @@ enum LeanShape : int { kLean96 = 0, kLean160 = 1, kLean256 = 2, kLean128 = 3, kL
 //   cs =  60, 2.5k blocks (M <=  74):   0.51 / 0.46 / 0.47 / 0.46 / 0.59
 //   cs = 100, 2.5k blocks (M <= 114):   1.10 / 0.96 / 0.93 / 0.98 / 1.27
 //   cs = 200, 2.5k blocks (M <= 214):   5.43 / 3.23 / 3.01 / 3.91 / 4.34
-inline int lean_table(int gen, int max_m, size_t blocks)
+inline int lean_table(int gen, int max_m, size_t blocks, int sms)
 {
-    const bool few = blocks <= 2 * 148;
+    const bool few = blocks <= 2 * (size_t)sms;
     if (gen == kGenXYZ) return (max_m <= 90 && !few) ? kLean128 : kLean256;
     if (max_m > 250) return kLean256;
     if (few) return kLean160Wide;

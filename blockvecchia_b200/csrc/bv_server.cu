@@ -403,7 +403,7 @@ struct LeanLaunch {
 
 bool lean_launch_for(const bv_server *S, int gen, int max_m, size_t blocks, LeanLaunch &ll)
 {
-    ll.v = &kLeanServer[lean_table(gen, max_m, blocks)];
+    ll.v = &kLeanServer[lean_table(gen, max_m, blocks, S->sms)];
     ll.smem = std::max<size_t>(lean_smem(gen, max_m, 0, S->lean_avail), kReduceScratchBytes);
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ll.v->kernel[gen], ll.v->threads, ll.smem) != cudaSuccess ||
