@@ -608,8 +608,11 @@ def run_ours(args):
         serve.pop("clocks", None)
 
     # FP64: fused kernel + reduction; mixed: probe, decision, mixed pass,
-    # FP64 fallback pass, reduction.
-    launches_per_eval = int(st["launches"])
+    # FP64 fallback pass, reduction.  The status leaves out the parameters'
+    # set-up kernel and, for a general nu on the streamed kernel, its table's.
+    launches_per_eval = int(st["launches"]) + 1
+    if w["nu"] not in (0.5, 1.5, 2.5) and int(st.get("streamed_blocks", 0)) > 0:
+        launches_per_eval += 1
     value = args.steps / (ms / 1e3)
     out = {
         "metric": METRIC,

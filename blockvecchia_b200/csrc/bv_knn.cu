@@ -503,7 +503,10 @@ __global__ void __launch_bounds__(kKnnWarps * 32) knn_kernel(KnnArgs a)
                 if (overflow) break;
                 __syncwarp();
                 // Distance to the nearest side that has cells beyond it, less
-                // the rounding of the cell assignment.
+                // the rounding of the cell assignment.  A side's coordinate is
+                // rounded once and rounding is monotone, so a location beyond
+                // the side is at or beyond its rounded coordinate too, however
+                // coarse coordinates are against the cells.
                 double d = INFINITY;
                 if (x0 > 0) d = fmin(d, cx - (g.x0 + x0 * g.hx) - 1e-6 * g.hx);
                 if (x1 < g.nx - 1) d = fmin(d, (g.x0 + (x1 + 1) * g.hx) - cx - 1e-6 * g.hx);

@@ -4,10 +4,12 @@
 // llh_Xvecchia_batch<double> (include/llh_Xvecchia_batch.h:22-522) and the
 // device allocations of its driver (src/test_Xvecchia_batch.cpp:459-600).
 // Layout data (locations, observations, conditioning indices) is copied to
-// HBM once at bv_create; one evaluation moves 48 bytes of parameters in and
-// one result record out, and runs as a CUDA graph:
-//   H2D params -> zero work counter -> fused per-block kernel(s)
-//   -> deterministic reduction -> D2H result.
+// HBM once at bv_create; an evaluation's parameters and its result record pass
+// through pinned host memory that the device reads and writes, and it runs as
+// a CUDA graph of kernels only (one graph for the closed forms of nu, one for
+// any other):
+//   parameters in, work counters zeroed -> (general nu) its table
+//   -> fused per-block kernel(s) -> deterministic reduction, result out.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -125,9 +127,9 @@ struct LeanVariant {
     {{llh_lean_kernel_t<NT, MINB, kGenClosed>, llh_lean_kernel_t<NT, MINB, kGenGeneral>,          \
       llh_lean_kernel_t<NT, MINB, kGenXYZ>}, NT}
 // In the order of LeanShape, and one more for the tuner: 256 x 1 is up to 2%
-// faster than 256 x 2 for a few blocks of M ~ 520 and more (cs = 500, 2k blocks
-// 8.69 against 8.83 ms; cs = 700, 150 blocks 3.47 / 3.48) and slower below (cs
-// = 300, 20k blocks 24.6 / 17.0).  In its place the one-warp kernel, where that
+// faster than 256 x 2 at M ~ 520 (cs = 500, 2k blocks 8.69 against 8.83 ms),
+// even at ~720 (cs = 700, 1.5k blocks 21.85 / 21.71) and slower below (cs = 300,
+// 20k blocks 24.6 / 17.0).  In its place the one-warp kernel, where that
 // applies (warp_variant).  All give the same bits, so bv_opts.tune may pick any.
 static const LeanVariant kLeanVariants[] = {
     BV_LEAN(96, 5), BV_LEAN(160, 3), BV_LEAN(256, 2), BV_LEAN(128, 4), BV_LEAN(160, 2), BV_LEAN(256, 1),
@@ -518,8 +520,8 @@ static int plan_lean_launch(bv_handle *h, const cudaDeviceProp &prop, int begin,
 
 // Which kernel evaluates which blocks.  Blocks are in the processing order
 // (largest first).  Under the default schedule every block whose two panels
-// fit the multi-CTA streamed kernel's shared memory (M up to ~780) runs that
-// kernel (several blocks per SM, so their pivot chains overlap); larger ones
+// fit the multi-CTA streamed kernel's shared memory (M up to 819, with a third
+// coordinate 797) runs that kernel (several blocks per SM, so their pivot chains overlap); larger ones
 // run the persistent one-CTA-per-SM kernel on a global slab.  The split
 // depends on the layout only, so every shard and every evaluation make the
 // same choice.

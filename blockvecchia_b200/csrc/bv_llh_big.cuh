@@ -214,11 +214,11 @@ __device__ __forceinline__ void panel_update_tiles(double *dst, int dst_r0, cons
 
 // Substitution rows of the factor warp per panel: with up to 256 rows below
 // the diagonal block (every panel of M <= ~290) warp 0 solves them all while
-// the other warps generate and update the next panel.  Kernel ms for n = 1M,
-// cs = 200 / n = 200k, cs = 120 / n = 20k, cs = 300: 32 rows 51.0 / 3.89 /
-// 1.91, 64 rows 50.4 / 3.87 / 1.89, 128 rows 49.7 / 3.78 / 1.86, 256 rows
-// 49.2 / 3.77 / 1.84 (rows dealt over the whole CTA after a barrier: 51.2 /
-// 3.84 / 1.92).
+// the other warps generate and update the next panel.  Streamed kernel's ms for
+// n = 1M, cs = 200 / n = 200k, cs = 120 / n = 20k, cs = 300 / 200k clustered,
+// cs = 300, nu = 0.8: 32 rows 34.96 / 2.51 / 1.49 / 21.2, 64 rows 34.53 / 2.47 /
+// 1.48 / 21.1, 128 rows 34.06 / 2.43 / 1.46 / 20.9, 256 rows 33.90 / 2.43 /
+// 1.45 / 20.8.
 constexpr int kSubstRows0 = 256;
 
 // One block by the streamed path, run by a CTA of NT threads (warp 0

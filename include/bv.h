@@ -93,13 +93,13 @@ typedef struct {
     int print_iter;    /* print the reference's per-evaluation line           */
     int use_graph;     /* capture one evaluation in a CUDA graph (default 1)  */
     int schedule;      /* BV_SCHED_AUTO (default): every block whose panels
-                          fit (M = cs + bs up to ~780) on the multi-CTA
-                          streamed kernel (several blocks per SM), larger
-                          ones on the persistent one-CTA-per-SM kernel;
+                          fit (M = cs + bs up to 819, with a third coordinate
+                          or earth 797) on the multi-CTA streamed kernel
+                          (several blocks per SM), larger ones on the persistent one-CTA-per-SM kernel;
                           BV_SCHED_BUCKETED: the persistent kernel, one
                           launch per size bucket (the comparison baseline);
                           BV_SCHED_PERSISTENT: the persistent kernel for
-                          every block (the server's algorithm);
+                          every block;
                           BV_SCHED_STREAMED: the streamed kernel for every
                           block (an error if one does not fit).  The two
                           kernels round differently; each choice depends on
