@@ -46,16 +46,15 @@ def test_deep_third_coordinate_cost(bvlib):
     x, y, z = _groups(300000, g, 1000.0)
     far = x.copy()
     far[0] = 1e12
-    best = []
-    for a in (x, far):
-        L = _layout3(bvlib, a, y, z, 100)
-        bvlib.knn(L)
-        t = []
-        for _ in range(9):
+    L = [_layout3(bvlib, a, y, z, 100) for a in (x, far)]
+    best = [np.inf, np.inf]
+    for rep in range(60):  # in turn, the least of each: the machine is shared
+        for i in (0, 1):
             t0 = time.perf_counter()
-            bvlib.knn(L)
-            t.append(time.perf_counter() - t0)
-        best.append(min(t))
+            bvlib.knn(L[i])
+            best[i] = min(best[i], time.perf_counter() - t0)
+        if rep >= 7 and best[0] <= 1.95 * best[1]:
+            break
     assert best[0] <= 1.95 * best[1], best
 
 
